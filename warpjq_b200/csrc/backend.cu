@@ -97,6 +97,7 @@ struct RunBufs {
   DevBuf<unsigned long long> row_off, line_idx;
   DevBuf<unsigned long long> block_lines;
   DevBuf<uint32_t> deep;
+  DevBuf<TemplateBuf> tmpl;  // a line template per plan of the run
   // group table
   DevBuf<unsigned long long> g_slots;
   DevBuf<GroupKeyDesc> g_keys;
@@ -122,14 +123,15 @@ struct RunBufs {
     b_tickets.release();
     b_rec_cursor.release();
     recs.release(); out.release(); row_off.release(); line_idx.release();
-    block_lines.release(); deep.release(); g_slots.release();
+    block_lines.release(); deep.release(); tmpl.release(); g_slots.release();
     g_keys.release(); g_acc.release();
   }
 };
 
 constexpr unsigned kReduceBlocks = 256;
 
-__global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, uint32_t key_cap) {
+__global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, uint32_t key_cap, TemplateBuf *tmpl,
+                            uint32_t n_tmpl) {
   unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   if (tid == 0) {
@@ -142,6 +144,7 @@ __global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, uint
     z.first_invalid = ~0ull;
     *ctr = z;
   }
+  for (unsigned long long i = tid; i < n_tmpl; i += stride) tmpl[i].state = tmpl[i].tries = 0;
   if (g.slots) {
     for (unsigned long long i = tid; i < g_cap; i += stride) g.slots[i] = 0;
     for (unsigned long long i = tid; i < key_cap; i += stride) group_acc_init(g.acc[i]);
@@ -430,7 +433,9 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     }
   }
   GroupTable g = group_view(rb, groups);
-  k_reset_run<<<256, 256, 0, st>>>(rb.ctr.p, g, groups ? rb.g_cap : 0, groups ? rb.g_key_cap : 0);
+  const uint32_t n_tmpl = b && b->mixed ? (uint32_t)b->plans.size() : 1u;
+  CK(rb.tmpl.ensure(n_tmpl, st, capturing), "alloc line templates");
+  k_reset_run<<<256, 256, 0, st>>>(rb.ctr.p, g, groups ? rb.g_cap : 0, groups ? rb.g_key_cap : 0, rb.tmpl.p, n_tmpl);
   s.kernels++;
   CK(cudaGetLastError(), "launch reset");
   if (n > 0 && n_tiles > 0) {
@@ -449,6 +454,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     sp.deep_words = rb.deep.p;
     sp.deep_levels_per_cta = rb.deep_levels;
     sp.rec_stride = run_rec_stride(c, b);
+    sp.tmpl = rb.tmpl.p;
     if (b && b->mixed) {
       sp.any_rows = b->any_rows ? 1u : 0u;
       CK(rb.b_tickets.ensure(b->plans.size(), st, capturing), "alloc batch tickets");
@@ -485,6 +491,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
         spk.tile_list = rb.b_plan_tiles.p + b->plan_tile0[k];
         spk.n_list = n_k;
         spk.ticket = rb.b_tickets.p + k;
+        spk.tmpl = rb.tmpl.p + k;
         spk.rec_cursor = Pk.needs_rows ? rb.b_rec_cursor.p : nullptr;
         const unsigned vg = Pk.needs_rows ? c->grid_rows : gk ? c->grid_group : c->grid_agg;
         const unsigned gr = (unsigned)std::min<unsigned long long>(vg, n_k);
@@ -653,6 +660,7 @@ uint64_t bufs_signature(const warpjq_ctx *c) {
   mix((uintptr_t)rb.row_off.p); mix((uintptr_t)rb.line_idx.p);
   mix((uintptr_t)rb.block_lines.p);
   mix((uintptr_t)rb.deep.p); mix(rb.deep.n);
+  mix((uintptr_t)rb.tmpl.p); mix(rb.tmpl.n);
   mix((uintptr_t)rb.g_slots.p); mix((uintptr_t)rb.g_keys.p); mix((uintptr_t)rb.g_acc.p);
   mix(rb.rec_cap_per_cta); mix(rb.out_cap); mix(rb.rows_cap); mix(rb.g_cap); mix(rb.g_key_cap);
   mix(rb.deep_levels); mix(c->tile_bytes); mix(c->halo_bytes); mix(c->grid); mix(c->scan_smem);

@@ -68,13 +68,14 @@ __device__ __forceinline__ uint32_t swar_movemask(uint32_t m) {
 
 // Exact per-byte flags (0x80 in each byte lane) of the bytes of x that are
 // '"', '\\' or below 0x20.  Each test adds to the low seven bits, which never
-// carries across a byte lane; bytes >= 0x80 are never flagged.
+// carries across a byte lane; bytes >= 0x80 are never flagged.  Flipping bit
+// 1 moves '"' (0x22) next to the control bytes, so one sum tests both: t is
+// below 0x21 for exactly those.
 __host__ __device__ __forceinline__ uint32_t flags_special(uint32_t x) {
-  const uint32_t t = x & 0x7F7F7F7Fu;
-  const uint32_t sq = (t ^ 0x22222222u) + 0x7F7F7F7Fu;  // bit 7 clear iff '"'
-  const uint32_t sb = (t ^ 0x5C5C5C5Cu) + 0x7F7F7F7Fu;  // bit 7 clear iff '\\'
-  const uint32_t sc = t + 0x60606060u;                  // bit 7 clear iff < 0x20
-  return ~((sq & sb & sc) | x) & 0x80808080u;
+  const uint32_t t = (x ^ 0x02020202u) & 0x7F7F7F7Fu;
+  const uint32_t sq = t + 0x5F5F5F5Fu;                  // bit 7 clear iff '"' or < 0x20
+  const uint32_t sb = (t ^ 0x5E5E5E5Eu) + 0x7F7F7F7Fu;  // bit 7 clear iff '\\'
+  return ~((sq & sb) | x) & 0x80808080u;
 }
 
 // Exact per-byte flags of the '\n' bytes of x.
@@ -220,6 +221,7 @@ __device__ inline int cmp_str_body(const uint8_t *body, uint32_t n, bool has_esc
                                    const uint8_t *lit, uint32_t lit_len) {
   if (!has_escape) {
     uint32_t m = n < lit_len ? n : lit_len;
+#pragma unroll 1
     for (uint32_t k = 0; k < m; k++) {
       uint32_t a = body[k], b = lit[k];
       if (a != b) return a < b ? -1 : 1;
@@ -228,6 +230,7 @@ __device__ inline int cmp_str_body(const uint8_t *body, uint32_t n, bool has_esc
   }
   StrDecoder d(body, n);
   uint32_t k = 0;
+#pragma unroll 1
   for (;;) {
     int a = d.next();
     if (a < 0) return k == lit_len ? 0 : -1;
@@ -241,6 +244,7 @@ __device__ inline int cmp_str_body(const uint8_t *body, uint32_t n, bool has_esc
 __device__ inline uint32_t hash_str_body(const uint8_t *body, uint32_t n, bool has_escape) {
   uint32_t h = 0x811c9dc5u;
   if (!has_escape) {
+#pragma unroll 1
     for (uint32_t k = 0; k < n; k++) {
       h ^= body[k];
       h *= 0x01000193u;
@@ -248,6 +252,7 @@ __device__ inline uint32_t hash_str_body(const uint8_t *body, uint32_t n, bool h
     return h;
   }
   StrDecoder d(body, n);
+#pragma unroll 1
   for (int c; (c = d.next()) >= 0;) {
     h ^= (uint32_t)c;
     h *= 0x01000193u;
@@ -257,6 +262,7 @@ __device__ inline uint32_t hash_str_body(const uint8_t *body, uint32_t n, bool h
 
 __device__ inline uint32_t hash_raw(const uint8_t *p, uint32_t n) {
   uint32_t h = 0x811c9dc5u;
+#pragma unroll 1
   for (uint32_t k = 0; k < n; k++) {
     h ^= p[k];
     h *= 0x01000193u;
@@ -284,6 +290,7 @@ __device__ __forceinline__ double exact_pow10(int e) {
   // 10^0 .. 10^22 are exact doubles.
   double r = 1.0;
   double b = 10.0;
+#pragma unroll 1
   while (e) {
     if (e & 1) r *= b;
     b *= b;
@@ -502,6 +509,7 @@ __device__ __forceinline__ double parse_number(const uint8_t *p, uint32_t n, boo
   if (n <= 9) {  // exact in 32 bits
     uint32_t v = 0;
     uint32_t k = 0;
+#pragma unroll 1
     for (; k < n; k++) {
       uint32_t dgt = (uint32_t)p[k] - '0';
       if (dgt > 9) break;
@@ -521,6 +529,7 @@ __device__ __forceinline__ double parse_number(const uint8_t *p, uint32_t n, boo
   bool dropped = false;    // a digit did not fit in mant
   bool overflow = false;   // a nonzero digit did not fit in mant
   // integer part
+#pragma unroll 1
   for (; i < n && is_digit(p[i]); i++) {
     uint32_t dgt = p[i] - '0';
     if (nd < 19) {
@@ -536,6 +545,7 @@ __device__ __forceinline__ double parse_number(const uint8_t *p, uint32_t n, boo
   if (i < n && p[i] == '.') {
     frac = true;
     i++;
+#pragma unroll 1
     for (; i < n && is_digit(p[i]); i++) {
       uint32_t dgt = p[i] - '0';
       if (nd < 19) {
@@ -557,6 +567,7 @@ __device__ __forceinline__ double parse_number(const uint8_t *p, uint32_t n, boo
       i++;
     }
     int e = 0;
+#pragma unroll 1
     for (; i < n && is_digit(p[i]); i++)
       if (e < 100000) e = e * 10 + (int)(p[i] - '0');
     exp10 += eneg ? -e : e;

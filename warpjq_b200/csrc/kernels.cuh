@@ -7,11 +7,11 @@
 //   k_scan      One warp per CTA.  A warp takes the next tile from a work
 //               ticket and stages tile + halo into shared memory with one
 //               bulk (TMA) copy.  Stage 1 is lane-parallel over 32-byte
-//               chunks: each chunk becomes two bit masks, its newlines and
-//               its "special" bytes ('"', '\\', < 0x20).  The lines that
-//               start in the tile are listed from the newline masks, and
-//               stage 2 walks them one line per lane (walker.cuh), jumping
-//               through strings by the special mask: validation, path
+//               chunks: each chunk's "special" bytes ('"', '\\', < 0x20)
+//               become a bit mask, its newlines line starts.  Stage 2 walks
+//               the lines one per lane (walker.cuh), by the run's line
+//               template where it fits, else from special byte to special
+//               byte of the mask: validation, path
 //               resolution, the filter, and either the aggregate or a
 //               compact record per selected row (line offset, row length,
 //               field spans).
@@ -37,12 +37,14 @@ namespace wjq {
 constexpr int kThreads = 32;                 // one warp per CTA; each warp owns its tile
 constexpr uint32_t kMaxLinesPerPass = 128;   // line-start list capacity per pass
 constexpr int kReduceThreads = 128;          // block size of the per-tile reductions
-// Register budgets of k_scan (warps per SM), measured per variant on the
-// nginx workload: the ungrouped aggregate at 24 (80 registers; more warps
-// hide more latency than its few spills cost), the row variant at 20 (96
-// registers, which keep its record writing from spilling) and the group-by
-// variants at 16 (128 registers).
-constexpr int kScanBlocksPerSM = 24;
+// Register budgets of k_scan (CTAs of one warp per SM), measured per variant
+// on 1 GB of the nginx workload: the ungrouped aggregate at 20 (96 registers,
+// 8 bytes of spills: 685 us; at 24, with 144 bytes, 713; at 16, 775), the row
+// variant at 20 and the group-by variant at 16 (128).  What the warps have in
+// common is the instruction cache: the body's loops are kept rolled and the
+// rare walks out of line, which took the same scan from 840 us to 685 with the
+// same work (misses had kept the next cache level 56% busy; 34% then).
+constexpr int kScanBlocksPerSM = 20;
 constexpr int kScanBlocksPerSMRows = 20;
 constexpr int kScanBlocksPerSMGrouped = 16;
 
@@ -55,28 +57,30 @@ constexpr int kGroupCache = 16;  // per-CTA group accumulators kept in shared me
 // the CTA (or of each tile, in a batch).
 struct CtaAcc {
   unsigned long long lines, blank, invalid, type, sel;
-  unsigned long long count, numeric, n_int;
+  unsigned long long numeric, n_int;
   unsigned long long isum_lo, isum_hi;  // exact 128-bit sum of the integer values
   unsigned long long min_bits, max_bits;
   uint32_t saw;  // a selected line had a non-numeric, non-null value
   uint32_t pad;
   __device__ void clear() {
-    lines = blank = invalid = type = sel = count = numeric = n_int = isum_lo = isum_hi = 0;
+    lines = blank = invalid = type = sel = numeric = n_int = isum_lo = isum_hi = 0;
     min_bits = ~0ull;
     max_bits = 0;
     saw = 0;
   }
 };
 
+static_assert(sizeof(CtaAcc) % 16 == 0, "the template after it is 16-byte aligned");
+
 // Readable bytes kept past a window's data: the end sentinel, the walker's
 // word reads after a line's newline, and the last chunk's 32-byte read.
 constexpr uint32_t kWinSlack = 64;
 
 // Shared-memory layout of k_scan for tile T and halo H: the window bytes,
-// then the special and newline masks (one word per 32-byte chunk, the
-// sentinel's chunk included), the CTA's exact FP sum, the mbarrier the
-// tile copies complete on, the line-start list, and for grouped aggregates
-// the group cache.  Nothing is static, so the dynamic size may be raised
+// then the special mask (one word per 32-byte chunk, the sentinel's chunk and
+// one more included), the CTA's exact FP sum, its counts, the line template,
+// the mbarrier the tile copies complete on, the line-start list, and for
+// grouped aggregates the group cache.  Nothing is static, so the dynamic size may be raised
 // to the device's whole opt-in limit.
 __host__ __device__ inline uint32_t scan_win_bytes(uint32_t T, uint32_t H) {
   return (T + H + kWinSlack + 15u) & ~15u;
@@ -86,9 +90,10 @@ __host__ __device__ inline uint32_t scan_chunk_words(uint32_t T, uint32_t H) {
 }
 __host__ __device__ inline size_t scan_smem_base(uint32_t T, uint32_t H) {
   size_t s = scan_win_bytes(T, H);
-  s += 2 * (size_t)scan_chunk_words(T, H) * sizeof(uint32_t);
+  s += (size_t)scan_chunk_words(T, H) * sizeof(uint32_t);
   s += kFixDigits * sizeof(long long);
   s += sizeof(CtaAcc);
+  s += sizeof(Template);
   s += sizeof(unsigned long long);  // the mbarrier of the tile copies
   s += (kMaxLinesPerPass + 2) * sizeof(uint16_t);
   return (s + 15) & ~(size_t)15;
@@ -180,6 +185,19 @@ struct RowTile {
   uint32_t pad;
 };
 
+// A run's line template in device memory (one per plan of a mixed batch):
+// made by the first CTA that can from a line it walked, taken over by the
+// others as they see it.  It only decides how fast a line is walked, so no
+// result depends on who made it, when, or from which line.
+struct TemplateBuf {
+  uint32_t state;  // kTmpl*, set to kTmplNone before the run
+  uint32_t tries;  // lines that had no template
+  Template t;
+};
+constexpr uint32_t kTmplNone = 0, kTmplBuilding = 1, kTmplReady = 2, kTmplOff = 3;
+constexpr uint32_t kTmplTries = 4;   // lines tried before the run goes on without one
+constexpr uint32_t kTmplMisses = 3;  // rounds that missed a line, past every second one, before a CTA stops using it
+
 struct ScanParams {
   const uint8_t *data;
   unsigned long long n;
@@ -217,6 +235,7 @@ struct ScanParams {
   unsigned long long n_list;
   unsigned long long *ticket;
   unsigned long long *rec_cursor;
+  TemplateBuf *tmpl;  // the run's line template (null: none is used)
 };
 
 // Rows emission.
@@ -262,11 +281,13 @@ __device__ __forceinline__ bool key_bytes_equal(const KeyRef &a, const uint8_t *
                                                 uint8_t besc) {
   if (!a.esc && !besc) {
     if (a.len != blen) return false;
+#pragma unroll 1
     for (uint32_t k = 0; k < blen; k++)
       if (a.p[k] != bp[k]) return false;
     return true;
   }
   StrDecoder x(a.p, a.len), y(bp, blen);
+#pragma unroll 1
   for (;;) {
     int u = x.next(), w = y.next();
     if (u != w) return false;
@@ -280,6 +301,7 @@ __device__ uint32_t group_find_or_insert(const ScanParams &sp, const KeyRef &k, 
   const GroupTable &g = sp.g;
   uint32_t pos = h & g.cap_mask;
   uint32_t mine = 0xFFFFFFFFu;
+#pragma unroll 1
   for (uint32_t probe = 0; probe <= g.cap_mask; probe++) {
     unsigned long long w = *(volatile unsigned long long *)&g.slots[pos];
     if (w == 0) {
@@ -325,6 +347,7 @@ __device__ __forceinline__ uint32_t csv_cell_len(const uint8_t *p, uint32_t n, b
   uint32_t len = 0, quotes = 0;
   bool need = false;
   if (!decode) {
+#pragma unroll 1
     for (uint32_t k = 0; k < n; k++) {
       uint32_t c = p[k];
       if (c == '"') quotes++;
@@ -333,6 +356,7 @@ __device__ __forceinline__ uint32_t csv_cell_len(const uint8_t *p, uint32_t n, b
     len = n;
   } else {
     StrDecoder d(p, n);
+#pragma unroll 1
     for (int c; (c = d.next()) >= 0;) {
       len++;
       if (c == '"') quotes++;
@@ -350,17 +374,20 @@ __device__ __forceinline__ uint32_t csv_cell_write(uint8_t *dst, const uint8_t *
   if (!decode) bare = n;
   else {
     StrDecoder d(p, n);
+#pragma unroll 1
     while (d.next() >= 0) bare++;
   }
   bool quote = expect_len != bare;
   if (quote) dst[w++] = '"';
   if (!decode) {
+#pragma unroll 1
     for (uint32_t k = 0; k < n; k++) {
       if (quote && p[k] == '"') dst[w++] = '"';
       dst[w++] = p[k];
     }
   } else {
     StrDecoder d(p, n);
+#pragma unroll 1
     for (int c; (c = d.next()) >= 0;) {
       if (quote && c == '"') dst[w++] = '"';
       dst[w++] = (uint8_t)c;
@@ -405,6 +432,7 @@ __device__ __forceinline__ uint32_t row_length(const DevPlan &P, const uint8_t *
 // before storing them, so one step moves 128 bytes with the loads in flight
 // together (lanes stride by 32: coalesced accesses).
 __device__ __forceinline__ void warp_copy(uint8_t *dst, const uint8_t *src, uint32_t n, int lane) {
+#pragma unroll 1
   for (uint32_t base = 0; base < n; base += 128) {
     const uint32_t k0 = base + lane;
     uint8_t b0 = 0, b1 = 0, b2 = 0, b3 = 0;
@@ -589,24 +617,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
   return false;
 }
 
-// 16-byte global -> shared copy that does not go through registers; bytes
-// past `src_bytes` (0..16) are zero-filled and not read.
-__device__ __forceinline__ void cp_async16(void *dst, const void *src, uint32_t src_bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(d), "l"(src), "r"(src_bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.wait_all;\n" ::: "memory");
-}
-
-__device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long x) {
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
-  return x;
-}
-
 // Exclusive warp scan of (a, b) in lane order, with the warp totals.
 __device__ __forceinline__ void warp_scan2(uint32_t a, unsigned long long b, uint32_t &ea,
                                            unsigned long long &eb, uint32_t &ta,
@@ -646,7 +656,7 @@ __device__ __noinline__ void flush_counts(RunCounters *dst, RunCounters *also, c
       if (acc->sel) atomicAdd(&c->n_selected, acc->sel);
     }
     if (!rows && P.group_slot < 0 && P.output_kind == 3) {
-      if (acc->count) atomicAdd(&dst->agg_count, acc->count);
+      if (acc->sel) atomicAdd(&dst->agg_count, acc->sel);  // an ungrouped aggregate counts every selected line
       if (acc->numeric) atomicAdd(&dst->agg_numeric, acc->numeric);
       if (acc->n_int) atomicAdd(&dst->agg_n_int, acc->n_int);
       const unsigned long long lo = acc->isum_lo, hi = acc->isum_hi;
@@ -684,10 +694,10 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   const uint32_t nwords = scan_chunk_words(T, H);
   uint8_t *win = smem;                                              // window bytes (+ slack)
   uint32_t *smask = (uint32_t *)(smem + scan_win_bytes(T, H));      // special bytes per chunk
-  uint32_t *nlmask = smask + nwords;                                // newlines per chunk
-  long long *cta_fix = (long long *)(nlmask + nwords);              // the CTA's exact FP sum
+  long long *cta_fix = (long long *)(smask + nwords);               // the CTA's exact FP sum
   CtaAcc *acc = (CtaAcc *)(cta_fix + kFixDigits);                   // the CTA's counts and aggregate
-  unsigned long long *s_bar = (unsigned long long *)(acc + 1);       // tile copies' mbarrier
+  Template *tmpl = (Template *)(acc + 1);                           // the run's line template, once seen
+  unsigned long long *s_bar = (unsigned long long *)(tmpl + 1);      // tile copies' mbarrier
   uint16_t *lstart = (uint16_t *)(s_bar + 1);                       // kMaxLinesPerPass + 2
   GroupCache *gcache = (GroupCache *)(smem + scan_smem_base(T, H));  // grouped aggregates only
 
@@ -707,6 +717,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   if (lane == 0) acc->clear();
   const bool grouped = kGroups && !kRows && P.group_slot >= 0;
   if (grouped) {
+#pragma unroll 1
     for (int k = lane; k < kGroupCache; k += 32) {
       gcache->tag[k] = 0xFFFFFFFFu;
       group_acc_init(gcache->acc[k]);
@@ -716,18 +727,22 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   if (lane == 0) mbar_init(bar);
   __syncwarp();
   uint32_t phase = 0;  // parity of the barrier's current phase
+  // What this CTA last saw of the run's template, and the rounds that missed
+  // a line by it, less half of all rounds since.
+  uint32_t tstate = sp.tmpl ? kTmplNone : kTmplOff, tmisses = 0;
 
-  // Tickets are taken one tile ahead, so the atomic's latency overlaps a
-  // tile's work.
+  // The first tile is the CTA's own; the others' tickets are taken one tile
+  // ahead, so the atomic's latency overlaps a tile's work.  (With every
+  // ticket from the counter, the CTAs that start first take two tiles each
+  // of an input with one per CTA, and the others none.)
   unsigned long long *const ticket_ctr = sp.ticket ? sp.ticket : &sp.ctr->next_tile;
-  unsigned long long next_ticket = 0;
-  if (lane == 0) next_ticket = atomicAdd(ticket_ctr, 1ull);
+  unsigned long long next_ticket = blockIdx.x;
   const unsigned long long n_work = sp.tile_list ? sp.n_list : sp.n_tiles;
   for (;;) {
     const unsigned long long ticket = __shfl_sync(0xffffffffu, next_ticket, 0);
     if (ticket >= n_work) break;
     const unsigned long long tile = sp.tile_list ? sp.tile_list[ticket] : ticket;
-    if (lane == 0) next_ticket = atomicAdd(ticket_ctr, 1ull);
+    if (lane == 0) next_ticket = gridDim.x + atomicAdd(ticket_ctr, 1ull);
     // The tile's input: the whole data, or one input of a batch (a window
     // never reaches past its input's end).
     uint32_t input = 0;
@@ -745,6 +760,11 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
     const uint32_t tlen = (uint32_t)(te - ts);
     const uint32_t wlen = (uint32_t)min((unsigned long long)T + H, data_end - ts);
     const bool win_reaches_end = ts + wlen == data_end;
+
+    // The run's template, until this CTA has it or the run goes without.
+    uint32_t tsee = 0;
+    if (tstate < kTmplReady && lane == 0)
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(tsee) : "l"(&sp.tmpl->state) : "memory");
 
     // 1. Stage tile + halo: the window's 16-byte multiple by one bulk copy
     //    (inputs and tiles start 16-byte aligned), its last 0-15 bytes by
@@ -765,44 +785,45 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       phase ^= 1u;
     }
     if (lane == 0 && win_reaches_end) win[wlen] = '\n';  // ends the last line for the walker
+    if (tstate < kTmplReady) {
+      tstate = __shfl_sync(0xffffffffu, tsee, 0);
+      if (tstate == kTmplReady)
+#pragma unroll 1
+        for (uint32_t k = lane; k < sizeof(Template) / 4; k += 32)
+          ((uint32_t *)tmpl)[k] = __ldcg((const uint32_t *)&sp.tmpl->t + k);
+    }
     __syncwarp();
 
     // 2. Stage 1, lane-parallel: every 32-byte chunk of the window (the end
-    //    sentinel's too) becomes its special and newline masks; lane l owns
-    //    chunks [l*K, l*K + K) and counts the line starts among them.
+    //    sentinel's too) becomes its special mask; lane l owns chunks
+    //    [l*K, l*K + K) and notes the newlines among them that start a line of
+    //    the tile, up to eight positions in one word each (the last ones
+    //    found lowest).  Bytes past the window's data are stale: no walk gets
+    //    past its line's newline, so their mask bits are never looked at.
     const uint32_t limit = wlen + (win_reaches_end ? 1u : 0u);  // classified bytes
     const uint32_t nchunks = (limit + 31) >> 5;
     const uint32_t K = (nchunks + 31) >> 5;
     const uint32_t c0 = lane * K;
     const uint32_t nl_limit = tlen - 1;  // newlines below this start a line in the tile
+    // the newlines of chunk c that start a line of the tile
     auto listed = [&](uint32_t c, uint32_t m) -> uint32_t {
-      const uint32_t base = c * 32;
-      if (base >= nl_limit) return 0u;
-      if (nl_limit - base < 32) m &= (1u << (nl_limit - base)) - 1u;
-      return m;
+      const uint32_t left = c * 32 < nl_limit ? nl_limit - c * 32 : 0u;
+      return left >= 32 ? m : m & ((1u << left) - 1u);
     };
     uint32_t my_nl = 0;
-    unsigned long long nz = 0;  // bit k: chunk c0 + k lists a line start
-    for (uint32_t k = 0; k < K; k++) {
-      const uint32_t c = c0 + k;
-      if (c >= nchunks) break;
+    unsigned long long nl_pos = 0;  // positions within the lane's chunks, 8 bits each
+    const uint32_t c1 = min(c0 + K, nchunks);
+#pragma unroll 1
+    for (uint32_t c = c0; c < c1; c++) {
       const uint4 u = ((const uint4 *)win)[2 * c];
       const uint4 v = ((const uint4 *)win)[2 * c + 1];
       const uint32_t w8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
       uint32_t sm_c;
-      uint32_t nl_c = classify_chunk(w8, &sm_c);
-      const uint32_t rem = limit - c * 32;
-      if (rem < 32) {  // bytes past the window's data are stale
-        sm_c &= (1u << rem) - 1u;
-        nl_c &= (1u << rem) - 1u;
-      }
+      uint32_t m = listed(c, classify_chunk(w8, &sm_c));
       smask[c] = sm_c;
-      nlmask[c] = nl_c;
-      const uint32_t lm = listed(c, nl_c);
-      if (lm) {
-        my_nl += __popc(lm);
-        nz |= 1ull << k;
-      }
+      my_nl += __popc(m);
+#pragma unroll 1
+      for (; m; m &= m - 1u) nl_pos = nl_pos << 8 | ((c - c0) * 32u + (uint32_t)__ffs(m) - 1u);
     }
 
     // The next tile's window is fetched into L2 now (its ticket has
@@ -823,114 +844,177 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
 
     // 3. Lines starting in the tile: ts itself (after a newline) and q+1 for
     //    every newline q in [ts, te-1).
-    uint32_t first_nl, tot_nl;
-    unsigned long long dummy_e, dummy_t;
-    warp_scan2(my_nl, 0ull, first_nl, dummy_e, tot_nl, dummy_t);
+    uint32_t first_nl = my_nl;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t x = __shfl_up_sync(0xffffffffu, first_nl, d);
+      if (lane >= d) first_nl += x;
+    }
+    const uint32_t tot_nl = __shfl_sync(0xffffffffu, first_nl, 31);
+    first_nl -= my_nl;
     const uint32_t lead = prev_nl;
     const uint32_t n_lines_tile = tot_nl + lead;
+    // whether every lane's newlines are noted (else they are found again)
+    const bool noted = K <= 8 && !__any_sync(0xffffffffu, my_nl > 8);
+    // The tile's last line ends at the first newline at or after te - 1 (the
+    // sentinel's, when the window reaches the data's end): looked for 512
+    // bytes at a time, 16 a lane.
+    uint32_t last_end = 0xFFFFFFFFu;  // none: the line is longer than the window
+#pragma unroll 1
+    for (uint32_t base = nl_limit & ~15u; base < limit && last_end == 0xFFFFFFFFu; base += 512) {
+      const uint32_t at = base + 16 * lane;
+      uint32_t first = 0xFFFFFFFFu;
+      if (at < limit) {
+        const uint4 u = *(const uint4 *)(win + at);
+        uint32_t m = flags_push(flags_push(flags_push(flags_push(0, flags_newline(u.w)), flags_newline(u.z)),
+                                           flags_newline(u.y)), flags_newline(u.x));
+        if (at < nl_limit) m &= 0xFFFFFFFFu << (nl_limit - at);
+        if (limit - at < 16) m &= (1u << (limit - at)) - 1u;
+        if (m) first = at + (uint32_t)__ffs(m) - 1u;
+      }
+      last_end = __reduce_min_sync(0xffffffffu, first);
+    }
 
     // 4. Walk the lines, one per lane, in passes of the list's capacity.
     unsigned long long tile_rows = 0, tile_bytes = 0;
     const unsigned long long tile_rec0 = cta_recs;
-    uint32_t tile_first_invalid = 0xFFFFFFFFu, tile_first_type = 0xFFFFFFFFu;
+    uint32_t tile_first_invalid = 0xFFFFFFFFu, tile_first_type = 0xFFFFFFFFu, tile_sel = 0;
+#pragma unroll 1
     for (uint32_t base = 0; base < n_lines_tile; base += kMaxLinesPerPass) {
       const uint32_t cnt = min(n_lines_tile - base, kMaxLinesPerPass);
       // list line starts [base, base + cnt] (one extra as the end marker)
       if (lead && lane == 0 && base == 0) lstart[0] = 0;
       {
-        uint32_t idx = first_nl + lead;
-        if (my_nl && idx <= base + cnt && idx + my_nl > base) {
-          for (unsigned long long z = nz; z; z &= z - 1) {
-            const uint32_t k = (uint32_t)__ffsll((long long)z) - 1u;
-            uint32_t m = listed(c0 + k, nlmask[c0 + k]);
-            while (m) {
-              uint32_t b = (c0 + k) * 32 + (uint32_t)__ffs(m) - 1;
-              m &= m - 1;
-              if (idx >= base && idx <= base + cnt) lstart[idx - base] = (uint16_t)(b + 1);
-              idx++;
-            }
+        const uint32_t idx = first_nl + lead;  // of this lane's first newline
+        if (noted) {
+#pragma unroll 1
+          for (uint32_t k = 0; k < my_nl; k++) {
+            const uint32_t i = idx + my_nl - 1u - k - base;
+            if (i <= cnt) lstart[i] = (uint16_t)(c0 * 32u + ((uint32_t)(nl_pos >> (8 * k)) & 0xFFu) + 1u);
+          }
+        } else if (my_nl && idx <= base + cnt && idx + my_nl > base) {
+          uint32_t i = idx - base;  // wraps below the pass
+#pragma unroll 1
+          for (uint32_t c = c0; c < c1; c++) {
+            const uint4 u = ((const uint4 *)win)[2 * c];
+            const uint4 v = ((const uint4 *)win)[2 * c + 1];
+            const uint32_t w8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+            uint32_t unused;
+#pragma unroll 1
+            for (uint32_t m = listed(c, classify_chunk(w8, &unused)); m; m &= m - 1u, i++)
+              if (i <= cnt) lstart[i] = (uint16_t)(c * 32u + (uint32_t)__ffs(m));
           }
         }
       }
       __syncwarp();
+#pragma unroll 1
       for (uint32_t b0 = 0; b0 < cnt; b0 += 32) {
         const uint32_t li = b0 + lane;  // line index within the pass
         int status = -1;
         uint32_t has_row = 0, row_len = 0;
-        unsigned long long line_abs = 0;
-        uint32_t line_len = 0, ordinal = base + li;
+        const uint32_t ordinal = base + li;
+        uint32_t s = 0, e = 0;  // window offsets of the line and of its newline
+        bool found = false;     // the line lies in the window
         const uint8_t *lp = nullptr;
+        uint32_t line_len = 0;
         bool has_group = false;
         KeyRef gk;
         uint32_t gh = 0;
         SlotVal aggv;
         aggv.kind = JK_MISSING;
         if (li < cnt) {
-          uint32_t s = lstart[li];
-          uint32_t e;  // window offset of the newline (or of the data end)
-          bool found = true;
-          if (base + li + 1 < n_lines_tile) {
-            // the next line's start is listed (the list keeps one entry past
-            // the pass for exactly this)
-            e = (uint32_t)lstart[li + 1] - 1;
-          } else {
-            // last line of the tile: its newline is at or after te - 1 (the
-            // sentinel's, when the window reaches the data's end)
-            uint32_t q = tlen - 1;
-            if (q < s) q = s;
-            uint32_t c = q >> 5;
-            uint32_t m = c < nchunks ? (nlmask[c] & (0xFFFFFFFFu << (q & 31))) : 0u;
-            while (!m && ++c < nchunks) m = nlmask[c];
-            if (m) e = c * 32 + (uint32_t)__ffs(m) - 1;
-            else found = false;
-          }
-          line_abs = ts + s;
-          if (found) {
-            lp = win + s;
-            line_len = e - s;
-            status = walk_objects(P, win, smask, s, e, nv);
-            if (status == LS_FALLBACK) status = walk_masked(P, win, smask, s, e, nv);
-          } else {
+          s = lstart[li];
+          // the next line's start is listed (the list keeps one entry past
+          // the pass for exactly this), except after the tile's last line
+          e = base + li + 1 < n_lines_tile ? (uint32_t)lstart[li + 1] - 1u : last_end;
+          found = e != 0xFFFFFFFFu;
+        }
+        const unsigned long long line_abs = ts + s;
+
+        // The walk.  A slot's value ends up in slots[]; bad_slots says which
+        // of them are type errors (resolve_slots).
+        uint32_t bad_slots = 0;
+        bool walk = found;  // not decided by the template
+        if (tstate == kTmplReady) {
+          SlotVal none;
+          none.off = none.len = 0;
+          none.state = SS_MISSING;
+          none.kind = JK_MISSING;
+          none.esc = 0;
+#pragma unroll 1
+          for (uint32_t k = 0; k < P.n_slots; k++) slots[k] = none;
+          const int st = walk_template(tmpl, win, smask, s, e, found, slots);  // every lane
+          walk = found && st != LS_OK;
+          if (found) status = LS_OK;
+        }
+        if (found) {
+          lp = win + s;
+          line_len = e - s;
+        }
+        // Everything below, to the next bracket, is for lines no template fits.
+        if (__any_sync(0xffffffffu, walk || (li < cnt && !found))) {
+          const bool far = li < cnt && !found;
+          const int st = walk_objects(P, win, smask, s, e, nv, walk);  // every lane
+          if (walk) status = st == LS_FALLBACK ? walk_masked(P, win, smask, s, e, nv) : st;
+          if (far) {
             // longer than the window: walk it from global memory
             unsigned long long q = ts + wlen;
+#pragma unroll 1
             while (q < data_end && sp.data[q] != '\n') q++;
             lp = sp.data + line_abs;
             line_len = (uint32_t)(q - line_abs);
             status = walk_line(P, lp, line_len, nv, nullptr);
           }
-        }
-        // Lines nesting past 64 levels share this CTA's deep stack, so they
-        // are walked one at a time.
-        if (__any_sync(0xffffffffu, status == LS_DEEP)) {
-          for (int t = 0; t < 32; t++) {
-            if (lane == t && status == LS_DEEP) {
-              status = walk_line(P, lp, line_len, nv, &deep);
-              if (status == LS_DEEP_FULL) {
-                atomicOr(&sp.ctr->overflow, 8u);
-                status = LS_INVALID;
+          __syncwarp();
+          const unsigned ok = __ballot_sync(0xffffffffu, walk && status == LS_OK);
+          if (tstate == kTmplReady) {
+            // a template that most rounds miss a line of costs more than it saves
+            if (ok && (tmisses += 2) > 2 * kTmplMisses) tstate = kTmplOff;
+          } else if (tstate == kTmplNone) {
+            // one line is enough, and only a CTA with another tile to walk tries
+            const bool more = __shfl_sync(0xffffffffu, next_ticket < n_work ? 1u : 0u, 0);
+            if (ok && more) {
+              tstate = kTmplBuilding;  // by this CTA or another: looked up at the next tile
+              if (lane == __ffs(ok) - 1 && atomicCAS(&sp.tmpl->state, kTmplNone, kTmplBuilding) == kTmplNone) {
+                uint32_t next = kTmplReady;
+                if (!build_template(P, win, smask, s, e, tmpl))
+                  next = ++sp.tmpl->tries < kTmplTries ? kTmplNone : kTmplOff;
+                else
+                  sp.tmpl->t = *tmpl;
+                __threadfence();
+                atomicExch(&sp.tmpl->state, next);
               }
             }
-            __syncwarp();
           }
+          // Lines nesting past 64 levels share this CTA's deep stack, so they
+          // are walked one at a time.
+          if (__any_sync(0xffffffffu, status == LS_DEEP)) {
+#pragma unroll 1
+            for (int t = 0; t < 32; t++) {
+              if (lane == t && status == LS_DEEP) {
+                status = walk_line(P, lp, line_len, nv, &deep);
+                if (status == LS_DEEP_FULL) {
+                  atomicOr(&sp.ctr->overflow, 8u);
+                  status = LS_INVALID;
+                }
+              }
+              __syncwarp();
+            }
+          }
+          if ((walk || far) && status == LS_OK) bad_slots = resolve_slots(P, nv, slots);
+          __syncwarp();
         }
-        // `line_len` for output excludes a trailing '\r' (chunk.rs:433-435).
+        if (tmisses) tmisses--;
+        // `out_len`: the line without a trailing '\r' (chunk.rs:433-435).
         uint32_t out_len = line_len;
         if (status >= 0 && out_len && lp[out_len - 1] == '\r') out_len--;
 
         if (status == LS_OK) {
-          uint32_t type_err_filter = 0, type_err_post = 0;
-          for (uint32_t s = 0; s < P.n_slots; s++) {
-            slots[s] = resolve_slot(P, nv, s);
-            if (slots[s].state == SS_TYPE_ERROR) {
-              if ((P.filter_slot_mask >> s) & 1) type_err_filter = 1;
-              else type_err_post = 1;
-            }
-          }
-          if (type_err_filter) {
+          if (bad_slots & 1u) {
             status = LS_TYPE_ERROR;
-          } else if (P.has_filter && !eval_filter(P, lp, slots)) {
+          } else if (P.has_filter && !(found ? eval_filter_win(P, win, s, slots) : eval_filter_far(P, lp, slots))) {
             status = 100;  // filtered out
-          } else if (type_err_post) {
+          } else if (bad_slots) {
             status = LS_TYPE_ERROR;
           } else {
             status = 101;  // selected
@@ -984,7 +1068,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
         bool saw = false;
         if (contrib && P.agg_slot >= 0) {
           if (aggv.kind == JK_NUM) {
-            fv = parse_number(lp + aggv.off, aggv.len, is_int, iv);
+            fv = found ? detail::parse_number_win(win, s + aggv.off, aggv.len, is_int, iv)
+                       : detail::parse_number_far(lp + aggv.off, aggv.len, is_int, iv);
             is_num = true;
           } else if (aggv.kind != JK_MISSING && aggv.kind != JK_NULL) {
             saw = true;
@@ -994,13 +1079,23 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
         // and added to the CTA's shared accumulator by lane 0.
         {
           const unsigned full = 0xffffffffu;
-          const unsigned m_blank = __ballot_sync(full, status == LS_BLANK);
-          const unsigned m_inv = __ballot_sync(full, status == LS_INVALID);
-          const unsigned m_type = __ballot_sync(full, status == LS_TYPE_ERROR);
+          if (__any_sync(full, status >= 0 && status < 100)) {  // neither selected nor filtered out
+            const unsigned m_blank = __ballot_sync(full, status == LS_BLANK);
+            const unsigned m_inv = __ballot_sync(full, status == LS_INVALID);
+            const unsigned m_type = __ballot_sync(full, status == LS_TYPE_ERROR);
+            if (lane == 0) {
+              acc->blank += __popc(m_blank);
+              acc->invalid += __popc(m_inv);
+              acc->type += __popc(m_type);
+            }
+          }
           const unsigned m_sel = __ballot_sync(full, status == 101);
+          tile_sel += __popc(m_sel);
+        }
+        if (!kRows && P.agg_slot >= 0 && __any_sync(0xffffffffu, contrib)) {
+          const unsigned full = 0xffffffffu;
           const unsigned m_saw = __ballot_sync(full, saw);
           const bool ung = contrib && !has_group;
-          const unsigned m_cnt = __ballot_sync(full, ung);
           const unsigned m_num = __ballot_sync(full, ung && is_num);
           const unsigned m_int = __ballot_sync(full, ung && is_num && is_int);
           unsigned long long s_lo = 0, s_hi = 0, ext = 0;
@@ -1012,13 +1107,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
           if (ung && is_num && !is_int && (ak == WARPJQ_AGG_SUM || ak == WARPJQ_AGG_AVG))
             fix_atomic_add(cta_fix, &ctr_in->fbig, fv);  // exact, in the CTA's shared limbs
           if (lane == 0) {
-            acc->blank += __popc(m_blank);
-            acc->invalid += __popc(m_inv);
-            acc->type += __popc(m_type);
-            acc->sel += __popc(m_sel);
             if (m_saw) acc->saw = 1;
-            if (m_cnt) {
-              acc->count += __popc(m_cnt);
+            if (m_num) {
               acc->numeric += __popc(m_num);
               acc->n_int += __popc(m_int);
               if (s_lo || s_hi) {
@@ -1026,8 +1116,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
                 acc->isum_lo = o + s_lo;
                 acc->isum_hi += s_hi + (acc->isum_lo < o ? 1ull : 0ull);
               }
-              if (m_num && ak == WARPJQ_AGG_MIN) acc->min_bits = min(acc->min_bits, ext);
-              if (m_num && ak == WARPJQ_AGG_MAX) acc->max_bits = max(acc->max_bits, ext);
+              if (ak == WARPJQ_AGG_MIN) acc->min_bits = min(acc->min_bits, ext);
+              if (ak == WARPJQ_AGG_MAX) acc->max_bits = max(acc->max_bits, ext);
             }
           }
         }
@@ -1112,6 +1202,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
               r->local_off = (uint32_t)(tile_bytes + eb);
               r->row_len = row_len;
               uint32_t *fl = (uint32_t *)(r + 1);
+#pragma unroll 1
               for (uint32_t f = 0; f < nf; f++) {
                 const SlotVal &s = slots[P.output_kind == 1 ? P.out_slot : P.field_slot[f]];
                 fl[2 * f] = s.off;
@@ -1128,7 +1219,10 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       }
       __syncwarp();
     }
-    if (lane == 0) acc->lines += n_lines_tile;
+    if (lane == 0) {
+      acc->lines += n_lines_tile;
+      acc->sel += tile_sel;
+    }
 
     // Per-tile bookkeeping.
     tile_first_invalid = __reduce_min_sync(0xffffffffu, tile_first_invalid);
@@ -1164,6 +1258,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   // Merge this CTA's cached group accumulators into the global records.
   if (grouped) {
     __syncwarp();
+#pragma unroll 1
     for (int k = lane; k < kGroupCache; k += 32) {
       const uint32_t kid = gcache->tag[k];
       if (kid == 0xFFFFFFFFu) continue;
@@ -1182,6 +1277,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
         atomicAdd(&a.n_int, c.n_int);
       }
       if (c.numeric > c.n_int) {
+#pragma unroll 1
         for (int d = 0; d < kFixDigits; d++)
           if (c.fix[d]) atomicAdd((unsigned long long *)&a.fix[d], (unsigned long long)c.fix[d]);
         if (c.fbig != 0.0) atomicAdd(&a.fbig, c.fbig);

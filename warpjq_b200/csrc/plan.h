@@ -59,6 +59,7 @@ struct PlanCmp {
   uint8_t op;        // WARPJQ_OP_*
   uint8_t lit_kind;  // WARPJQ_LIT_*
   uint8_t lit_rank;  // jq type rank of the literal (ir.rs:100-108)
+  uint32_t lit_w[2];  // a string literal's first 8 bytes, little-endian, zero past its end
 };
 
 struct PlanCond {

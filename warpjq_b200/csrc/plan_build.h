@@ -177,6 +177,10 @@ inline warpjq_status build_plan(const warpjq_program *p, DevPlan &P, char *err, 
     d.op = (uint8_t)c.op;
     d.lit_kind = (uint8_t)c.lit_kind;
     d.lit_rank = (uint8_t)c.lit_kind;  // null 0, false 1, true 2, num 3, str 4 (ir.rs:100-108)
+    d.lit_w[0] = d.lit_w[1] = 0;
+    if (c.lit_kind == 4)
+      for (uint32_t k = 0; k < 8 && k < c.lit_len; k++)
+        d.lit_w[k >> 2] |= (uint32_t)p->blob[c.lit_off + k] << (8 * (k & 3));
     P.filter_slot_mask |= 1u << s;
   }
   P.n_cond = p->n_cond;

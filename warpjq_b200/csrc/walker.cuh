@@ -63,8 +63,10 @@ __device__ __forceinline__ long long scan_string_bytes(const uint8_t *line, uint
                                                        bool &esc) {
   uint32_t j = s + 1;
   esc = false;
+#pragma unroll 1
   for (;;) {
     // Aligned word steps over runs of ordinary bytes.
+#pragma unroll 1
     while (((uintptr_t)(line + j) & 3u) == 0 && j + 4 <= n &&
            swar_string_special(*(const uint32_t *)(line + j)) == 0)
       j += 4;
@@ -107,17 +109,20 @@ __device__ __forceinline__ bool valid_atom(const uint8_t *p, uint32_t n) {
   if (p[i] == '0') {
     i++;
   } else {
+#pragma unroll 1
     while (i < n && is_digit(p[i])) i++;
   }
   if (i < n && p[i] == '.') {
     i++;
     if (i >= n || !is_digit(p[i])) return false;
+#pragma unroll 1
     while (i < n && is_digit(p[i])) i++;
   }
   if (i < n && (p[i] == 'e' || p[i] == 'E')) {
     i++;
     if (i < n && (p[i] == '+' || p[i] == '-')) i++;
     if (i >= n || !is_digit(p[i])) return false;
+#pragma unroll 1
     while (i < n && is_digit(p[i])) i++;
   }
   return i == n;
@@ -137,6 +142,7 @@ __device__ __forceinline__ uint8_t kind_of(uint32_t c) {
 // Key child of `node` whose decoded key equals the key body, or kNoNode.
 __device__ __forceinline__ uint8_t match_key(const DevPlan &P, uint8_t node, const uint8_t *body,
                                              uint32_t len, bool esc) {
+#pragma unroll 1
   for (uint8_t c = P.nodes[node].first_child; c != kNoNode; c = P.nodes[c].next_sibling) {
     const PlanNode &nd = P.nodes[c];
     if (nd.is_index) continue;
@@ -145,6 +151,7 @@ __device__ __forceinline__ uint8_t match_key(const DevPlan &P, uint8_t node, con
       if (len && body[0] != nd.key_first) continue;
       const uint8_t *k = P.blob + nd.key_off;
       uint32_t t = 1;
+#pragma unroll 1
       while (t < len && body[t] == k[t]) t++;
       if (t >= len) return c;
     } else if (cmp_str_body(body, len, true, P.blob + nd.key_off, nd.key_len) == 0) {
@@ -156,6 +163,7 @@ __device__ __forceinline__ uint8_t match_key(const DevPlan &P, uint8_t node, con
 
 __device__ __forceinline__ uint8_t index_child(const DevPlan &P, uint8_t node, uint32_t idx) {
   if (node == kNoNode || !P.nodes[node].has_index_children) return kNoNode;
+#pragma unroll 1
   for (uint8_t c = P.nodes[node].first_child; c != kNoNode; c = P.nodes[c].next_sibling) {
     const PlanNode &nd = P.nodes[c];
     if (nd.is_index && nd.index == idx) return c;
@@ -171,12 +179,15 @@ __device__ __noinline__ int walk_line(const DevPlan &P, const uint8_t *line, uin
                                       NodeVals &v, const DeepStack *deep) {
   using namespace detail;
   const uint32_t n_nodes = P.n_nodes;
+#pragma unroll 1
   for (uint32_t k = 0; k < n_nodes; k++) v.kind[k] = JK_MISSING;
 
   uint32_t i = 0;
+#pragma unroll 1
   while (i < n && is_ws(line[i])) i++;
   if (i == n) return LS_BLANK;
   if (line[i] == 0x0C) {  // form feed counts toward a blank line, not toward JSON
+#pragma unroll 1
     for (uint32_t j = i; j < n; j++) {
       uint32_t c = line[j];
       if (!(c == ' ' || c == '\t' || c == '\r' || c == 0x0C)) return LS_INVALID;
@@ -191,7 +202,9 @@ __device__ __noinline__ int walk_line(const DevPlan &P, const uint8_t *line, uin
   uint8_t pending = n_nodes ? 0 : kNoNode;  // node the next value lands on
   int expect = EX_VALUE;
 
+#pragma unroll 1
   for (;;) {
+#pragma unroll 1
     while (i < n && is_ws(line[i])) i++;
     if (i >= n) break;
     uint32_t c = line[i];
@@ -267,6 +280,7 @@ __device__ __noinline__ int walk_line(const DevPlan &P, const uint8_t *line, uin
     // A value starts at i (expect is EX_VALUE or EX_VALUE_OR_CLOSE).
     uint8_t vn = pending;
     if (vn != kNoNode) {
+#pragma unroll 1
       for (uint32_t k = vn + 1u; k < P.nodes[vn].subtree_end; k++) v.kind[k] = JK_MISSING;
       v.kind[vn] = kind_of(c);
       v.off[vn] = i;
@@ -304,6 +318,7 @@ __device__ __noinline__ int walk_line(const DevPlan &P, const uint8_t *line, uin
       if (vn != kNoNode) v.esc[vn] = esc;
     } else {
       uint32_t j = i + 1;
+#pragma unroll 1
       while (j < n && !ends_atom(line[j])) j++;
       if (!valid_atom(line + i, j - i)) return LS_INVALID;
       vend = j;
@@ -327,8 +342,15 @@ namespace detail {
 __device__ __forceinline__ bool is_ws3(uint32_t c) { return c == ' ' || c == '\t' || c == '\r'; }
 
 __device__ __forceinline__ uint32_t skip_ws3(const uint8_t *w, uint32_t i) {
+#pragma unroll 1
   while (is_ws3(w[i])) i++;
   return i;
+}
+
+// Index of the lowest set bit of a nonzero word.
+__device__ __forceinline__ uint32_t low_bit64(unsigned long long x) {
+  const uint32_t lo = (uint32_t)x;
+  return lo ? (uint32_t)__ffs(lo) - 1u : 31u + (uint32_t)__ffs((uint32_t)(x >> 32));
 }
 
 // Four bytes at any offset of a 4-byte-aligned window.
@@ -341,12 +363,13 @@ __device__ __forceinline__ uint32_t load4(const uint8_t *w, uint32_t i) {
 // them.
 __device__ __forceinline__ uint32_t digit_run(const uint8_t *w, uint32_t j, uint32_t &term) {
   uint32_t n = 0;
+#pragma unroll 1
   for (;;) {
     uint32_t x = load4(w, j + n);
-    // a byte is a digit when its high nibble is 3 and its low nibble is <= 9
-    uint32_t nd = ((x & 0xF0F0F0F0u) ^ 0x30303030u) | (((x & 0x0F0F0F0Fu) + 0x06060606u) & 0x10101010u);
+    // flags the bytes that are no digit: x ^ '0' is at most 9 for a digit
+    const uint32_t nd = ((((x ^ 0x30303030u) & 0x7F7F7F7Fu) + 0x76767676u) | x) & 0x80808080u;
     if (nd) {
-      const uint32_t sh = ((uint32_t)__ffs(nd) - 1u) & ~7u;
+      const uint32_t sh = (uint32_t)__ffs(nd) - 8u;
       term = (x >> sh) & 0xFFu;
       return n + (sh >> 3);
     }
@@ -354,9 +377,63 @@ __device__ __forceinline__ uint32_t digit_run(const uint8_t *w, uint32_t j, uint
   }
 }
 
+// The value of a validated number too long or too odd for the window forms
+// below (signs, exponents, more than eight bytes).
+__device__ __noinline__ double parse_number_far(const uint8_t *p, uint32_t n, bool &is_int, long long &iv) {
+  return parse_number(p, n, is_int, iv);
+}
+
+// Four decimal digit values (the first digit in the low byte) as a number:
+// pairs by one multiply by 10, their sum by one multiply by 100.
+__device__ __forceinline__ uint32_t four_digits(uint32_t y) {
+  const uint32_t t = (y * 10u + (y >> 8)) & 0x00FF00FFu;
+  return (t * 100u + (t >> 16)) & 0xFFFFu;
+}
+
+// parse_number for the n bytes at w[o, o + n) of a window (the 12 bytes from
+// o on readable): up to eight bytes of digits, with one '.' or none, take a
+// fixed number of steps for every lane, instead of one step a digit.
+__device__ __forceinline__ double parse_number_win(const uint8_t *w, uint32_t o, uint32_t n, bool &is_int,
+                                                   long long &iv) {
+  if (n <= 8) {
+    // the bytes xor '0' in the top n bytes of y, first byte lowest: zeros
+    // (the digit 0) before the first
+    const uint32_t x0 = load4(w, o) ^ 0x30303030u, x1 = load4(w, o + 4) ^ 0x30303030u;
+    unsigned long long y = ((unsigned long long)x1 << 32 | x0) << (64u - 8u * n);
+    const unsigned long long k7 = 0x7F7F7F7F7F7F7F7Full, k8 = 0x8080808080808080ull;
+    unsigned long long odd = (((y & k7) + 0x7676767676767676ull) | y) & k8;  // bytes that are no digit
+    uint32_t frac = 0;
+    if (odd && !(odd & (odd - 1))) {  // one of them: a '.' is taken out
+      const uint32_t at = low_bit64(odd) - 7u;  // its lowest bit
+      if (((y >> at) & 0xFFu) == ('.' ^ '0')) {
+        frac = 7u - (at >> 3);
+        const unsigned long long low = y & ((1ull << at) - 1ull);
+        y = (y & ~((2ull << (at + 7u)) - 1ull)) | low << 8;
+        odd = 0;
+      }
+    }
+    if (!odd) {
+      const uint32_t v = four_digits((uint32_t)y) * 10000u + four_digits((uint32_t)(y >> 32));
+      is_int = !frac;
+      iv = (long long)v;
+      // a fraction has at most seven digits before and after the '.': one
+      // correctly rounded division by an exact power of ten
+      return frac ? (double)v / exact_pow10((int)frac) : (double)v;
+    }
+  }
+  return parse_number_far(w + o, n, is_int, iv);
+}
+
+// One of " \ / b f n r t: a bit per letter, the letters' columns 0x20-0x3F,
+// 0x40-0x5F and 0x60-0x7F picked by their high bits.
 __device__ __forceinline__ bool simple_escape(uint32_t e) {
-  return e == '"' || e == '\\' || e == '/' || e == 'b' || e == 'f' || e == 'n' || e == 'r' ||
-         e == 't';
+  const uint32_t row = e >> 5;
+  const uint32_t set = row == 1 ? (1u << ('"' & 31) | 1u << ('/' & 31))
+                       : row == 2 ? 1u << ('\\' & 31)
+                       : row == 3 ? (1u << ('b' & 31) | 1u << ('f' & 31) | 1u << ('n' & 31) | 1u << ('r' & 31) |
+                                     1u << ('t' & 31))
+                                  : 0u;
+  return (set >> (e & 31u)) & 1u;
 }
 
 // Closing quote of the string opened at w[i], or 0 when the string is
@@ -370,9 +447,11 @@ __device__ __forceinline__ uint32_t mask_string(const uint8_t *w, const uint32_t
                                                 bool &esc) {
   uint32_t p = i + 1;
   esc = false;
+#pragma unroll 1
   for (;;) {
     uint32_t k = p >> 5;
     uint32_t m = sm[k] & (0xFFFFFFFFu << (p & 31u));
+#pragma unroll 1
     while (!m) m = sm[++k];
     p = (k << 5) + (uint32_t)__ffs(m) - 1u;
     const uint32_t c = w[p];
@@ -395,9 +474,12 @@ __device__ __forceinline__ uint32_t mask_string(const uint8_t *w, const uint32_t
 // End (exclusive) of the number or literal starting at w[i] == c, or 0 when
 // it is malformed.  The byte after it is checked by the caller.
 __device__ __forceinline__ uint32_t win_atom(const uint8_t *w, uint32_t i, uint32_t c) {
-  if (c == 't') return load4(w, i) == 0x65757274u ? i + 4 : 0;      // "true"
-  if (c == 'n') return load4(w, i) == 0x6C6C756Eu ? i + 4 : 0;      // "null"
-  if (c == 'f') return load4(w, i + 1) == 0x65736C61u ? i + 5 : 0;  // "alse"
+  if (c > '9') {
+    if (c == 't') return load4(w, i) == 0x65757274u ? i + 4 : 0;      // "true"
+    if (c == 'n') return load4(w, i) == 0x6C6C756Eu ? i + 4 : 0;      // "null"
+    if (c == 'f') return load4(w, i + 1) == 0x65736C61u ? i + 5 : 0;  // "alse"
+    return 0;
+  }
   // -?(0|[1-9][0-9]*)(\.[0-9]+)?([eE][+-]?[0-9]+)?   (json.rs:370-410)
   uint32_t j = i;
   if (c == '-') c = w[++j];
@@ -429,6 +511,7 @@ __device__ __forceinline__ uint8_t match_key_win(const DevPlan &P, uint8_t node,
   const uint32_t w0 = load4(w, off), w1 = load4(w, off + 4);
   const uint32_t m0 = len >= 4 ? 0xFFFFFFFFu : (1u << (8 * len)) - 1u;
   const uint32_t m1 = len >= 8 ? 0xFFFFFFFFu : len > 4 ? (1u << (8 * (len - 4))) - 1u : 0u;
+#pragma unroll 1
   for (uint8_t c = P.nodes[node].first_child; c != kNoNode; c = P.nodes[c].next_sibling) {
     const PlanNode &nd = P.nodes[c];
     if (nd.is_index || nd.key_len != len) continue;
@@ -436,6 +519,7 @@ __device__ __forceinline__ uint8_t match_key_win(const DevPlan &P, uint8_t node,
     if (len <= 8) return c;
     const uint8_t *k = P.blob + nd.key_off;
     uint32_t t = 8;
+#pragma unroll 1
     while (t < len && w[off + t] == k[t]) t++;
     if (t >= len) return c;
   }
@@ -453,6 +537,7 @@ __device__ __noinline__ int walk_masked(const DevPlan &P, const uint8_t *w, cons
                                            uint32_t s, uint32_t e, NodeVals &v) {
   using namespace detail;
   const uint32_t n_nodes = P.n_nodes;
+#pragma unroll 1
   for (uint32_t k = 0; k < n_nodes; k++) v.kind[k] = JK_MISSING;
 
   uint32_t i = s;
@@ -463,6 +548,7 @@ __device__ __noinline__ int walk_masked(const DevPlan &P, const uint8_t *w, cons
   }
   if (c == '\n') return LS_BLANK;
   if (c == 0x0C) {  // form feed counts toward a blank line, not toward JSON
+#pragma unroll 1
     for (; i < e; i++) {
       c = w[i];
       if (!(is_ws3(c) || c == 0x0C)) return LS_INVALID;
@@ -479,6 +565,7 @@ __device__ __noinline__ int walk_masked(const DevPlan &P, const uint8_t *w, cons
   uint32_t vn = n_nodes ? 0u : kNoNode;  // node the next value lands on
   bool want_key = false;
 
+#pragma unroll 1
   for (;;) {
     if (want_key) {
       if (c != '"') return LS_INVALID;
@@ -508,6 +595,7 @@ __device__ __noinline__ int walk_masked(const DevPlan &P, const uint8_t *w, cons
     }
     // A value starts at w[i] == c.
     if (vn != kNoNode) {
+#pragma unroll 1
       for (uint32_t k = vn + 1u; k < P.nodes[vn].subtree_end; k++) v.kind[k] = JK_MISSING;
       v.kind[vn] = kind_of(c);
       v.off[vn] = i - s;
@@ -553,6 +641,7 @@ __device__ __noinline__ int walk_masked(const DevPlan &P, const uint8_t *w, cons
     // After a value: commas and closing brackets, with the next bytes read
     // four at a time.
     uint32_t la = load4(w, i);
+#pragma unroll 1
     for (;;) {
       c = la & 0xFFu;
       if (is_ws3(c)) {
@@ -596,17 +685,32 @@ __device__ __forceinline__ bool hex4_at(const uint8_t *w, uint32_t i) {
   return hex_val(w[i]) >= 0 && hex_val(w[i + 1]) >= 0 && hex_val(w[i + 2]) >= 0 && hex_val(w[i + 3]) >= 0;
 }
 
-// Position of the next special byte (a set bit of the window's special mask)
-// from the cursor (k, m), consuming it.  The line's newline is special, so
-// a walk that reaches it stops there.
-__device__ __forceinline__ uint32_t pop_special(const uint32_t *sm, uint32_t &k, uint32_t &m) {
-  while (!m) m = sm[++k];
-  const uint32_t b = (k << 5) + (uint32_t)__ffs(m) - 1u;
-  m &= m - 1u;
-  return b;
+// Position of the first special byte at or after p (a set bit of the window's
+// special mask).  The line's newline is special, so no search from within a
+// line passes it.
+__device__ __forceinline__ uint32_t next_special(const uint32_t *sm, uint32_t p) {
+  for (;;) {
+    const uint32_t k = p >> 5, m = __funnelshift_r(sm[k], sm[k + 1], p & 31u);
+    if (m) return p + (uint32_t)__ffs(m) - 1u;
+    p += 32;
+  }
 }
 
 }  // namespace detail
+
+// The lanes of a warp meet here; whether any of them says so.
+__device__ __forceinline__ void warp_meet() {
+#ifdef __CUDA_ARCH__
+  __syncwarp();
+#endif
+}
+__device__ __forceinline__ bool warp_any(bool x) {
+#ifdef __CUDA_ARCH__
+  return __any_sync(0xffffffffu, x);
+#else
+  return x;
+#endif
+}
 
 // The fast path of the window walk, for the common shape of a log line: one
 // object whose members are separated by single ',' and ':' with no
@@ -615,24 +719,26 @@ __device__ __forceinline__ uint32_t pop_special(const uint32_t *sm, uint32_t &k,
 // to special byte: a key is its two quotes, a string value its quotes and
 // escapes, and only the bytes right after them are read ('"' ':' value, ','
 // or '}').  Lines of that shape get exactly walk_masked's verdict and node
-// values; a line it finds malformed where every check so far has passed (a
-// raw control byte or the line's end inside a string, a value that is no
-// number or literal) is LS_INVALID without the general walk; for any other
-// line (whitespace, arrays, escaped keys, deeper nesting, anything else
-// malformed) it returns LS_FALLBACK and records nothing that walk_masked
-// does not overwrite.  Same window contract as walk_masked.
+// values; a line that breaks off from it where nothing valid goes on is
+// LS_INVALID without the general walk; for any other line (whitespace, arrays,
+// empty objects, escaped keys, deeper nesting) it returns LS_FALLBACK and
+// records nothing that walk_masked does not overwrite.  (One line left to
+// walk_masked costs its warp a walk of its own, so malformed lines are worth
+// deciding here.)  Same window contract as walk_masked.
 //
-// Checks whose outcome does not steer the walk (that a key's quotes are
-// quotes where they were expected, the ':' after it, an escape's letter)
-// are folded into `bad` and decided once, when the line's object closes, so
-// the shared-memory loads behind them do not stall each step.  Every pop is
-// bounded by the line's newline (a special byte), so a walk over a line of
-// another shape still ends at e.
-__device__ __forceinline__ int walk_objects(const DevPlan &P, const uint8_t *w, const uint32_t *sm,
-                                            uint32_t s, uint32_t e, NodeVals &v) {
+// All lanes of a warp call it together, `on` where the lane has a line, and
+// take one member a turn: its key, then its value by kind, then the closing
+// brackets after it, meeting again after each (no lane leaves a turn early:
+// the compiler then runs the ones that stay apart from each other).  Lines
+// whose members come in different orders keep 22 of 32 lanes busy this way,
+// against 13 when each lane ran on by itself.
+__device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, const uint32_t *sm, uint32_t s,
+                                         uint32_t e, NodeVals &v, bool on = true) {
   using namespace detail;
-  if (w[s] != '{') return LS_FALLBACK;
   const uint32_t n_nodes = P.n_nodes;
+  int status = LS_FALLBACK;
+  on = on && w[s] == '{';
+#pragma unroll 1
   for (uint32_t k = 0; k < n_nodes; k++) v.kind[k] = JK_MISSING;
   uint32_t cur = n_nodes ? 0u : kNoNode;  // trie node of the innermost open object
   unsigned long long lm = 0;             // its key_len_mask (0: no key is looked up)
@@ -644,86 +750,113 @@ __device__ __forceinline__ int walk_objects(const DevPlan &P, const uint8_t *w, 
   }
   unsigned long long stack = 0;  // trie nodes of the enclosing objects, 8 bits a level
   uint32_t depth = 1;
-  uint32_t k = (s + 1) >> 5;
-  uint32_t m = sm[k] & (0xFFFFFFFFu << ((s + 1) & 31u));
   uint32_t p = s + 1;  // where the next key's opening quote must be
-  uint32_t bad = 0;    // deferred checks: nonzero when the line is not of this shape
-  for (;;) {
-    const uint32_t q0 = pop_special(sm, k, m);
-    if (q0 >= e) return LS_FALLBACK;
-    const uint32_t q1 = pop_special(sm, k, m);
-    if (q1 >= e) return LS_FALLBACK;
-    bad |= (q0 ^ p) | ((uint32_t)w[q0] ^ '"') | ((uint32_t)w[q1] ^ '"');
-    uint32_t vn = kNoNode;
-    const uint32_t kl = q1 - q0 - 1;
-    if ((lm >> (kl < 63u ? kl : 63u)) & 1ull) vn = match_key_win(P, (uint8_t)cur, w, q0 + 1, kl, false);
-    const uint32_t la = load4(w, q1 + 1);
-    bad |= (la & 0xFFu) ^ ':';
-    const uint32_t c = (la >> 8) & 0xFFu;
-    const uint32_t vs = q1 + 2;
-    if (vn != kNoNode) {
+  bool opened = true;  // just after a '{'
+  // a byte that cannot be here, unless it is whitespace: the line's verdict
+  auto broken = [&](uint32_t x) {
+    on = false;
+    if (!is_ws3(x)) status = LS_INVALID;
+  };
+  while (warp_any(on)) {
+    uint32_t vn = kNoNode, vs = 0, c = 0;
+    if (on && w[p] != '"') {
+      if (opened && w[p] == '}') on = false;
+      else broken(w[p]);
+    }
+    if (on) {
+      const uint32_t q = next_special(sm, p + 1);
+      const uint32_t la = load4(w, q + 1);
+      if (w[q] != '"') {  // an escape, or a byte below 0x20 (the newline among them)
+        on = false;
+        if (w[q] != '\\') status = LS_INVALID;
+      } else if ((la & 0xFFu) != ':') {
+        broken(la & 0xFFu);
+      }
+      vs = q + 2;
+      c = (la >> 8) & 0xFFu;
+      const uint32_t kl = q - p - 1;
+      if (on && ((lm >> (kl < 63u ? kl : 63u)) & 1ull)) vn = match_key_win(P, (uint8_t)cur, w, p + 1, kl, false);
+    }
+    warp_meet();
+    if (on && vn != kNoNode) {
+#pragma unroll 1
       for (uint32_t x = vn + 1u; x < P.nodes[vn].subtree_end; x++) v.kind[x] = JK_MISSING;
       v.kind[vn] = kind_of(c);
       v.off[vn] = vs - s;
       v.esc[vn] = 0;
     }
-    if (c == '{') {
-      if (depth >= 8) return LS_FALLBACK;
-      stack = (stack << 8) | cur;
-      depth++;
-      cur = vn;
-      lm = vn != kNoNode ? P.nodes[vn].key_len_mask : 0ull;
-      p = vs + 1;
-      continue;
-    }
-    uint32_t ve;
-    if (c == '"') {
-      const uint32_t r0 = pop_special(sm, k, m);  // the opening quote, at vs
-      if (r0 >= e) return LS_FALLBACK;
-      bad |= r0 ^ vs;
-      bool esc = false;
-      uint32_t r;
-      for (;;) {
-        r = pop_special(sm, k, m);
-        const uint32_t b = w[r];
-        if (b == '"') break;
-        // a raw control byte or the newline inside a string: with every
-        // earlier check passed, the line is malformed whatever its shape
-        if (b != '\\') return bad ? LS_FALLBACK : LS_INVALID;
-        esc = true;
-        const uint32_t x = w[r + 1];
-        if (x == '"' || x == '\\') {
-          pop_special(sm, k, m);  // the escaped byte is special itself (r + 1 < e)
-        } else if (x == 'u') {
-          bad |= hex4_at(w, r + 2) ? 0u : 1u;
+    uint32_t ve = 0;  // the value's end; 0 when an object was opened
+    bool go = on && c == '"', esc = false;
+    if (go) {
+      ve = vs + 1;
+#pragma unroll 1
+      while (go) {
+        const uint32_t k = ve >> 5, m = __funnelshift_r(sm[k], sm[k + 1], ve & 31u);
+        if (!m) {
+          ve += 32;
         } else {
-          bad |= simple_escape(x) ? 0u : 1u;  // a special x stops the next pop
+          ve += (uint32_t)__ffs(m) - 1u;
+          const uint32_t x = w[ve];
+          go = x == '\\';
+          if (go) {
+            const uint32_t y = w[ve + 1];
+            esc = true;
+            if (!simple_escape(y)) on = go = y == 'u' && hex4_at(w, ve + 2);
+            ve++;
+          } else {
+            on = x == '"';
+          }
+          ve++;
         }
       }
-      ve = r + 1;
-      if (vn != kNoNode) v.esc[vn] = esc;
-    } else {
-      if (c == '[') return LS_FALLBACK;
-      ve = win_atom(w, vs, c);
-      // no number or literal at the value's place (a bare word, a bad
-      // number, a cut literal): malformed, unless an earlier check failed
-      // or the value is only preceded by whitespace
-      if (!ve) return (bad || c == ' ' || c == '\t' || c == '\r') ? LS_FALLBACK : LS_INVALID;
+      if (!on) status = LS_INVALID;  // a control byte (the newline among them) or a bad escape
+      if (on && esc && vn != kNoNode) v.esc[vn] = 1;
     }
-    if (vn != kNoNode) v.len[vn] = ve - vs;
-    // after a value: ',' and the next key, or '}' closing one or more objects
-    uint32_t t = w[ve];
-    while (t == '}') {
-      if (cur != kNoNode) v.len[cur] = ve + 1 - s - v.off[cur];
-      if (--depth == 0) return (ve + 1 == e && !bad) ? LS_OK : LS_FALLBACK;
-      cur = (uint32_t)(stack & 0xFFu);
-      stack >>= 8;
-      lm = cur != kNoNode ? P.nodes[cur].key_len_mask : 0ull;
-      t = w[++ve];
+    warp_meet();
+    if (on && c != '"') {
+      if (c == '{') {
+        on = depth < 8;
+        stack = (stack << 8) | cur;
+        depth++;
+        cur = vn;
+        lm = vn != kNoNode ? P.nodes[vn].key_len_mask : 0ull;
+        p = vs + 1;
+        opened = true;
+      } else if (c == '[') {
+        on = false;
+      } else {
+        ve = win_atom(w, vs, c);
+        if (!ve) broken(c);
+      }
     }
-    if (t != ',') return LS_FALLBACK;
-    p = ve + 1;
+    warp_meet();
+    if (on && ve) {
+      if (vn != kNoNode) v.len[vn] = ve - vs;
+      // after a value: ',' and the next key, or '}' closing one or more objects
+      uint32_t t = w[ve];
+#pragma unroll 1
+      while (t == '}') {
+        ve++;
+        if (cur != kNoNode) v.len[cur] = ve - s - v.off[cur];
+        depth--;
+        cur = (uint32_t)(stack & 0xFFu);
+        stack >>= 8;
+        t = depth ? w[ve] : 0u;
+      }
+      if (!depth) {
+        on = false;
+        if (ve == e) status = LS_OK;
+        else if (!is_ws3(w[ve])) status = LS_INVALID;
+      } else if (t != ',') {
+        broken(t);
+      }
+      p = ve + 1;
+      opened = false;
+      lm = on && cur != kNoNode ? P.nodes[cur].key_len_mask : 0ull;
+    }
+    warp_meet();
   }
+  return status;
 }
 
 // ---------------------------------------------------------------------------
@@ -732,12 +865,12 @@ __device__ __forceinline__ int walk_objects(const DevPlan &P, const uint8_t *w, 
 
 enum SlotState : uint8_t { SS_FOUND = 0, SS_MISSING = 1, SS_TYPE_ERROR = 2 };
 
-struct SlotVal {
+struct alignas(16) SlotVal {  // one 16-byte load or store
+  uint32_t off;
+  uint32_t len;
   uint8_t state;  // SlotState
   uint8_t kind;   // JKind (JK_MISSING when not found)
   uint8_t esc;
-  uint32_t off;
-  uint32_t len;
 };
 
 // Resolves slot `s` from the node values (json.rs:461-507).  Walking up from
@@ -747,6 +880,7 @@ __device__ __forceinline__ SlotVal resolve_slot(const DevPlan &P, const NodeVals
   SlotVal r;
   uint8_t t = P.slot_node[s];
   uint8_t st = SS_FOUND;
+#pragma unroll 1
   for (uint8_t c = t; c != 0;) {
     uint8_t p = P.nodes[c].parent;
     uint8_t kp = v.kind[p];
@@ -821,6 +955,7 @@ __device__ __forceinline__ bool truthy(const uint8_t *line, const SlotVal &s) {
 __device__ __forceinline__ bool eval_filter(const DevPlan &P, const uint8_t *line,
                                             const SlotVal *slots) {
   uint64_t st = 0;  // bit stack, top at bit 0
+#pragma unroll 1
   for (uint32_t k = 0; k < P.n_cond; k++) {
     const PlanCond &o = P.cond[k];
     switch (o.op) {
@@ -848,6 +983,294 @@ __device__ __forceinline__ bool eval_filter(const DevPlan &P, const uint8_t *lin
     }
   }
   return st & 1;
+}
+
+// compare_slot for a line at w + s of a window (its number and string reads
+// stay in the window).
+__device__ __forceinline__ int compare_slot_win(const DevPlan &P, const uint8_t *w, uint32_t s, const SlotVal &v,
+                                                const PlanCmp &c) {
+  using namespace detail;
+  // the kinds from JK_NUM on are their jq ranks; null and missing rank 0
+  const uint32_t sr = v.kind == JK_BOOL ? (w[s + v.off] == 't' ? 2u : 1u) : v.kind <= JK_NULL ? 0u : v.kind;
+  if (sr != c.lit_rank) return sr < c.lit_rank ? -1 : 1;
+  if (c.lit_kind == 3 /* NUM */) {
+    bool is_int;
+    long long iv;
+    const double d = parse_number_win(w, s + v.off, v.len, is_int, iv);
+    return d < c.lit_num ? -1 : d > c.lit_num ? 1 : 0;
+  }
+  if (c.lit_kind == 4 /* STR */) {
+    const uint32_t o = s + v.off + 1, n = v.len - 2;
+    if (c.op <= 1 && !v.esc) {  // equality: the length, then the first eight bytes
+      if (n != c.lit_len) return 1;
+      const uint32_t m0 = n >= 4 ? 0xFFFFFFFFu : (1u << (8 * n)) - 1u;
+      const uint32_t m1 = n >= 8 ? 0xFFFFFFFFu : n > 4 ? (1u << (8 * (n - 4))) - 1u : 0u;
+      if ((load4(w, o) & m0) != c.lit_w[0] || (load4(w, o + 4) & m1) != c.lit_w[1]) return 1;
+      if (n <= 8) return 0;
+    }
+    return cmp_str_body(w + o, n, v.esc, P.blob + c.lit_off, c.lit_len);
+  }
+  return 0;
+}
+
+// eval_filter for a line at w + s of a window.
+__device__ __forceinline__ bool eval_filter_win(const DevPlan &P, const uint8_t *w, uint32_t s, const SlotVal *slots) {
+  uint64_t st = 0;  // bit stack, top at bit 0
+#pragma unroll 1
+  for (uint32_t k = 0; k < P.n_cond; k++) {
+    const PlanCond &o = P.cond[k];
+    if (o.op == 0) {
+      const PlanCmp &c = P.cmps[o.arg];
+      st = (st << 1) | (op_accepts(c.op, compare_slot_win(P, w, s, slots[c.slot], c)) ? 1u : 0u);
+    } else if (o.op == 1) {
+      st = (st << 1) | (truthy(w + s, slots[o.arg]) ? 1u : 0u);
+    } else if (o.op == 2 || o.op == 3) {
+      const uint64_t b = st & 1, a = (st >> 1) & 1;
+      st = (st >> 2 << 1) | (o.op == 2 ? a & b : a | b);
+    } else {
+      st ^= 1;
+    }
+  }
+  return st & 1;
+}
+
+// eval_filter out of line, for lines outside the window (long ones).
+__device__ __noinline__ bool eval_filter_far(const DevPlan &P, const uint8_t *line, const SlotVal *slots) {
+  return eval_filter(P, line, slots);
+}
+
+// The slots of a walked line: bit 0 of the result where one that the filter
+// reads is a type error, bit 1 where another is.
+__device__ __noinline__ uint32_t resolve_slots(const DevPlan &P, const NodeVals &v, SlotVal *slots) {
+  uint32_t bad = 0;
+#pragma unroll 1
+  for (uint32_t k = 0; k < P.n_slots; k++) {
+    slots[k] = resolve_slot(P, v, k);
+    if (slots[k].state == SS_TYPE_ERROR) bad |= ((P.filter_slot_mask >> k) & 1) ? 1u : 2u;
+  }
+  return bad;
+}
+
+// ---------------------------------------------------------------------------
+// Line templates: log lines of one source repeat the same text around their
+// values, so a line is mostly a comparison.
+//
+// A template is the text of one valid line with its scalar values taken out:
+// literal 0, value, literal 1, value, ..., last literal.  A literal holds
+// everything between two values -- punctuation, keys, whitespace, opened and
+// closed objects, and a string value's own quotes.  A line that consists of
+// the same literals with any string body or any number, true, false or null
+// at the values' places is valid JSON with the template line's structure, so
+// each value's trie node and the kind of every object node are the
+// template's.  Any other line is left to the walkers below it.
+//
+// What bounds the walk is instructions: walk_objects spends about 1,860 warp
+// instructions on a 228-byte access-log line, most of them finding and
+// checking keys and punctuation one member at a time; comparing them four
+// bytes at a time takes about a third of that.
+// ---------------------------------------------------------------------------
+
+constexpr uint32_t kTmplSteps = 24;       // steps per line
+constexpr uint32_t kTmplStepBytes = 16;   // literal bytes per step (a longer literal takes several)
+constexpr uint32_t kTmplNodes = 32;       // trie nodes of the plan
+
+enum TmplValue : uint32_t { TV_NONE = 0, TV_STR = 1, TV_ATOM = 2 };
+
+constexpr uint32_t kNoSlot = 0xFF;
+
+// One step: up to 16 literal bytes, compared as four words under a byte mask
+// (always four: a flat compare has no loop, and its loads are in flight
+// together), then a value or none.
+struct alignas(16) Template {
+  uint32_t lit[kTmplSteps][4];
+  uint32_t mask[kTmplSteps][4];
+  uint32_t desc[kTmplSteps];  // literal bytes (bits 0-7), TmplValue (8-15), the value's slot (16-23)
+  uint32_t n_steps;
+  uint32_t pad[3];
+};
+
+
+// Makes the template of the line w[s, e), which must be a valid one (same
+// window contract as walk_masked).  False when the line has none: no object,
+// arrays, duplicate wanted keys, an object as a wanted value, a scalar where
+// a wanted path goes on (whose slot is missing or a type error, depending on
+// the value), or too large.
+__device__ __noinline__ bool build_template(const DevPlan &P, const uint8_t *w, const uint32_t *sm, uint32_t s,
+                                            uint32_t e, Template *t) {
+  using namespace detail;
+  const uint32_t n_nodes = P.n_nodes;
+  if (n_nodes > kTmplNodes) return false;
+  uint8_t seen[kTmplNodes];  // kinds of the nodes met: JK_OBJ, else JK_NUM for any scalar
+#pragma unroll 1
+  for (uint32_t k = 0; k < n_nodes; k++) seen[k] = JK_MISSING;
+  uint32_t ns = 0, lit0 = s, depth = 0;
+  uint8_t stk[8];
+  uint32_t vn = n_nodes ? 0u : kNoNode;  // node of the next value
+  bool key = false;                     // a key (not a value) comes next
+  // the steps of the literal [lit0, end) and the value after it
+  auto close_literal = [&](uint32_t end, uint32_t value, uint32_t node) -> bool {
+    uint32_t at = lit0, slot = kNoSlot;
+#pragma unroll 1
+    for (uint32_t k = 0; k < P.n_slots && node != kNoNode; k++)
+      if (P.slot_node[k] == node) {
+        if (slot != kNoSlot) return false;
+        slot = k;
+      }
+    do {
+      if (ns >= kTmplSteps) return false;
+      const uint32_t nb = end - at < kTmplStepBytes ? end - at : kTmplStepBytes;
+#pragma unroll 1
+      for (uint32_t k = 0; k < 4; k++) {
+        const uint32_t m = nb >= 4 * k + 4 ? 0xFFFFFFFFu : nb <= 4 * k ? 0u : 0xFFFFFFFFu >> (8 * (4 * k + 4 - nb));
+        t->lit[ns][k] = load4(w, at + 4 * k) & m;
+        t->mask[ns][k] = m;
+      }
+      at += nb;
+      t->desc[ns++] = nb | (at == end ? value << 8 | slot << 16 : TV_NONE << 8 | kNoSlot << 16);
+    } while (at < end);
+    return true;
+  };
+#pragma unroll 1
+  for (uint32_t i = s; i < e;) {
+    const uint32_t c = w[i];
+    if (is_ws3(c) || c == ':') {
+      i++;
+    } else if (c == '{') {
+      if (depth >= 8) return false;
+      if (vn != kNoNode) {
+        if (seen[vn]) return false;
+        seen[vn] = JK_OBJ;
+#pragma unroll 1
+        for (uint32_t k = 0; k < P.n_slots; k++)
+          if (P.slot_node[k] == vn) return false;
+      }
+      stk[depth++] = (uint8_t)vn;
+      key = true;
+      i++;
+    } else if (c == '}') {
+      if (!depth) return false;
+      depth--;
+      i++;
+    } else if (c == ',') {
+      key = true;
+      i++;
+    } else if (c == '[' || c == ']' || !depth) {
+      return false;
+    } else if (key) {
+      bool esc;
+      const uint32_t q = mask_string(w, sm, i, esc);
+      if (c != '"' || !q) return false;
+      const uint32_t cur = stk[depth - 1];
+      vn = kNoNode;
+      if (cur != kNoNode && P.nodes[cur].has_key_children)
+        vn = match_key_win(P, (uint8_t)cur, w, i + 1, q - i - 1, esc);
+      key = false;
+      i = q + 1;
+    } else {
+      if (vn != kNoNode) {
+        if (seen[vn]) return false;
+        seen[vn] = JK_NUM;
+      }
+      uint32_t end;
+      if (c == '"') {
+        bool esc;
+        end = mask_string(w, sm, i, esc);
+        if (!close_literal(i + 1, TV_STR, vn)) return false;
+      } else {
+        end = win_atom(w, i, c);
+        if (!close_literal(i, TV_ATOM, vn)) return false;
+      }
+      if (!end) return false;
+      lit0 = i = end;
+      if (c == '"') i++;
+    }
+  }
+  if (depth || !close_literal(e, TV_NONE, kNoNode)) return false;
+  // every path runs through objects of the line up to its value, or to a
+  // member that is not there
+#pragma unroll 1
+  for (uint32_t k = 0; k < P.n_slots; k++)
+#pragma unroll 1
+    for (uint32_t c = P.slot_node[k]; c != 0; c = P.nodes[c].parent) {
+      const uint32_t kp = seen[P.nodes[c].parent];
+      if (kp != JK_MISSING && (kp != JK_OBJ || P.nodes[c].is_index)) return false;
+    }
+  t->n_steps = ns;
+  return true;
+}
+
+// Walks w[s, e) by the template t (same window contract as walk_masked):
+// LS_OK with the slots' values (those of the template's line; the caller
+// sets the others to missing), or LS_FALLBACK for a line of another shape,
+// malformed ones among them.  All lanes of the warp call it together, with
+// `on` where the lane has a line (the others read at the window's start):
+// the steps are the same for every lane, so their loads are broadcasts, and
+// the lanes meet again after every value (no lane leaves the loop alone, or
+// the compiler would let the others run on apart from it).  A lane never
+// steps past e, and reads at most 20 bytes from where it is.
+__device__ __forceinline__ int walk_template(const Template *t, const uint8_t *w, const uint32_t *sm, uint32_t s,
+                                             uint32_t e, bool on, SlotVal *slots) {
+  using namespace detail;
+  const uint32_t ns = t->n_steps;
+  uint32_t p = on ? s : 0;
+#pragma unroll 1
+  for (uint32_t j = 0; j < ns; j++) {
+    const uint32_t d = t->desc[j];
+    {
+      const uint32_t *q = (const uint32_t *)w + (p >> 2), *L = t->lit[j], *M = t->mask[j];
+      const uint32_t sh = (p & 3u) * 8u;
+      const uint32_t a = q[0], b = q[1], c = q[2], f = q[3], g = q[4];
+      const uint32_t bad = ((__funnelshift_r(a, b, sh) ^ L[0]) & M[0]) | ((__funnelshift_r(b, c, sh) ^ L[1]) & M[1]) |
+                           ((__funnelshift_r(c, f, sh) ^ L[2]) & M[2]) | ((__funnelshift_r(f, g, sh) ^ L[3]) & M[3]);
+      // no literal holds a newline, so one that fits ends at or before e
+      on = on && !bad;
+      if (on) p += d & 0xFFu;
+    }
+    if (!warp_any(on)) break;
+    const uint32_t value = (d >> 8) & 0xFFu, slot = (d >> 16) & 0xFFu, b = p;
+    bool esc = false;
+    if (value == TV_STR) {
+      // from special byte to special byte of the stage-1 mask, 32 bytes at
+      // a time, until one that is not an escape's backslash
+      bool go = on;
+#pragma unroll 1
+      while (go) {
+        const uint32_t k = p >> 5, m = __funnelshift_r(sm[k], sm[k + 1], p & 31u);
+        if (!m) {
+          p += 32;
+        } else {
+          p += (uint32_t)__ffs(m) - 1u;
+          const uint32_t c = w[p];
+          go = c == '\\';
+          on = go || c == '"';  // else a byte below 0x20, the newline among them
+          if (go) {
+            const uint32_t x = w[p + 1];
+            esc = true;
+            if (!simple_escape(x)) on = go = x == 'u' && hex4_at(w, p + 2);
+            p += 2;
+          }
+        }
+      }
+      warp_meet();
+    } else if (value == TV_ATOM) {
+      if (on) {
+        p = win_atom(w, b, w[b]);
+        on = p != 0;
+      }
+      warp_meet();
+    }
+    if (slot != kNoSlot && on) {
+      const uint32_t q = value == TV_STR ? 1u : 0u;  // a string's span includes its quotes
+      SlotVal r;
+      r.state = SS_FOUND;
+      r.kind = q ? (uint8_t)JK_STR : kind_of(w[b]);
+      r.esc = esc;
+      r.off = b - q - s;
+      r.len = p - b + 2 * q;
+      slots[slot] = r;
+    }
+  }
+  return on && p == e ? LS_OK : LS_FALLBACK;
 }
 
 }  // namespace wjq
