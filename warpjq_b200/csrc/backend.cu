@@ -192,7 +192,6 @@ struct warpjq_ctx {
   int device = 0;
   int num_sms = 0;
   DevPlan plan;
-  DevPlan *d_plan = nullptr;
   unsigned long long chunk_cap = 0;
   uint32_t tile_bytes = 6144;
   uint32_t halo_bytes = 2048;
@@ -288,7 +287,7 @@ warpjq_status ensure_bufs(warpjq_ctx *c, Slot &s, unsigned long long n,
   CK(rb.deep.ensure((size_t)c->grid * (rb.deep_levels / 32), st, cap), "alloc deep stack");
   if (rows) {
     CK(rb.row_tiles.ensure(n_tiles, st, cap), "alloc row tiles");
-    CK(rb.row_bsum.ensure(3 * ((n_tiles + 31) / 32), st, cap), "alloc row prefixes");
+    CK(rb.row_bsum.ensure(3 * ((n_tiles + 7) / 8), st, cap), "alloc row prefixes");
     // Records accumulate over all of a CTA's tiles: room for a row per KiB
     // of input, grown on overflow; output and row capacities follow the
     // input's size too (a larger input than the last does not overflow
@@ -527,7 +526,6 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
                                                       rb.rows_cap, rb.out_cap);
       EmitParams ep{};
       ep.data = d_data;
-      ep.plan = c->d_plan;
       ep.rec_stride = sp.rec_stride;
       if (b && b->mixed) {
         ep.plans = rb.b_plans.p;
@@ -546,7 +544,8 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
       ep.line_idx = rb.line_idx.p;
       ep.rows_cap = rb.rows_cap;
       ep.ctr = rb.ctr.p;
-      k_rows_emit<<<nb, kEmitThreads, 0, st>>>(ep);
+      if (b && b->mixed) k_rows_emit<true><<<nb, kEmitThreads, 0, st>>>(ep, P);
+      else k_rows_emit<false><<<nb, kEmitThreads, 0, st>>>(ep, P);
       s.kernels += 3;
       CK(cudaGetLastError(), "launch rows");
     }
@@ -739,8 +738,6 @@ warpjq_status warpjq_ctx_create(const warpjq_program *prog, uint64_t max_chunk_b
     uint64_t keep = 8ull << 30;
     CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "memory pool");
   }
-  CK(cudaMalloc((void **)&c->d_plan, sizeof(DevPlan)), "alloc plan");
-  CK(cudaMemcpy(c->d_plan, &c->plan, sizeof(DevPlan), cudaMemcpyHostToDevice), "upload plan");
   rc = configure_grid(c.get(), err, err_len);
   if (rc != WARPJQ_OK) return rc;
   c->chunk_cap = max_chunk_bytes;
@@ -789,7 +786,6 @@ void warpjq_ctx_destroy(warpjq_ctx *ctx) {
   cudaDeviceSynchronize();
   for (auto &s : ctx->slots) free_slot(s);
   free_slot(ctx->dev);
-  if (ctx->d_plan) cudaFree(ctx->d_plan);
   delete ctx;
 }
 

@@ -241,9 +241,8 @@ struct ScanParams {
 // Rows emission.
 struct EmitParams {
   const uint8_t *data;
-  const DevPlan *plan;
   // A mixed batch: tile t's rows are rendered by plans[in_plan[tile_input[t]]]
-  // (null otherwise).
+  // (null otherwise: the kernel's own plan).
   const DevPlan *plans;
   const uint32_t *in_plan;
   const uint32_t *tile_input;
@@ -428,117 +427,86 @@ __device__ __forceinline__ uint32_t row_length(const DevPlan &P, const uint8_t *
   }
 }
 
-// Warp-cooperative copy of n bytes: each lane loads four bytes 32 apart
-// before storing them, so one step moves 128 bytes with the loads in flight
-// together (lanes stride by 32: coalesced accesses).
-__device__ __forceinline__ void warp_copy(uint8_t *dst, const uint8_t *src, uint32_t n, int lane) {
+// Rows are copied by groups of kEmitLanes lanes, a row a group.
+constexpr uint32_t kEmitLanes = 8;
+
+// Copies n bytes with one group (lane g of it): whole aligned words of the
+// output, each from the two source words it straddles, four a lane in flight,
+// and single bytes at both ends.  No word past the source's last is read.
+__device__ __forceinline__ void group_copy(uint8_t *dst, const uint8_t *src, uint32_t n, uint32_t g) {
+  const uint32_t head = min(n, (uint32_t)(-(uintptr_t)dst & 3u));
+  const uint32_t sh = (uint32_t)((uintptr_t)(src + head) & 3u) * 8u;
+  const uint32_t *sw = (const uint32_t *)((uintptr_t)(src + head) & ~(uintptr_t)3);
+  uint32_t *dw = (uint32_t *)(dst + head);
+  // output word k needs source words k and k + 1, which must end within it
+  const uint32_t avail = (uint32_t)((uintptr_t)(src + n) - (uintptr_t)sw) / 4u;
+  const uint32_t words = avail > 1u && n > head ? min((n - head) / 4u, avail - 1u) : 0u;
 #pragma unroll 1
-  for (uint32_t base = 0; base < n; base += 128) {
-    const uint32_t k0 = base + lane;
-    uint8_t b0 = 0, b1 = 0, b2 = 0, b3 = 0;
-    if (k0 < n) b0 = src[k0];
-    if (k0 + 32 < n) b1 = src[k0 + 32];
-    if (k0 + 64 < n) b2 = src[k0 + 64];
-    if (k0 + 96 < n) b3 = src[k0 + 96];
-    if (k0 < n) dst[k0] = b0;
-    if (k0 + 32 < n) dst[k0 + 32] = b1;
-    if (k0 + 64 < n) dst[k0 + 64] = b2;
-    if (k0 + 96 < n) dst[k0 + 96] = b3;
+  for (uint32_t k0 = g; k0 < words; k0 += 4 * kEmitLanes) {
+    uint32_t x[4];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      const uint32_t k = k0 + j * kEmitLanes;
+      x[j] = k < words ? __funnelshift_r(__ldg(sw + k), __ldg(sw + k + 1), sh) : 0u;
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 4; j++) {
+      const uint32_t k = k0 + j * kEmitLanes;
+      if (k < words) dw[k] = x[j];
+    }
   }
+  if (g < head) dst[g] = src[g];
+#pragma unroll 1
+  for (uint32_t k = head + 4 * words + g; k < n; k += kEmitLanes) dst[k] = src[k];
 }
 
-// Segment s of a value or projection row (JSON output): the value of the
-// single path, or prefix 0, value 0, prefix 1, value 1, ..., then the
-// suffix; the last segment is the newline.
-__device__ __forceinline__ const uint8_t *row_segment(const DevPlan &P, const uint8_t *line,
-                                                      const uint32_t *fields, uint32_t nf,
-                                                      uint32_t s, uint32_t &len) {
-  const bool proj = P.output_kind == 2;
-  const uint32_t n_before_suffix = proj ? 2 * nf : nf;
-  if (s < n_before_suffix) {
-    const uint32_t f = proj ? s >> 1 : s;
-    if (proj && !(s & 1)) {
-      len = P.prefix_len[f];
-      return P.blob + P.prefix_off[f];
-    }
-    const uint32_t off = fields[2 * f], lk = fields[2 * f + 1];
-    if ((lk >> 28) == JK_MISSING) {
-      len = 4;
-      return (const uint8_t *)"null";
-    }
-    len = lk & 0x07FFFFFFu;
-    return line + off;
-  }
-  if (proj && s == n_before_suffix) {
-    len = P.suffix_len;
-    return P.blob + P.suffix_off;
-  }
-  len = 1;
-  return (const uint8_t *)"\n";
-}
-
-// Writes one row.  All lanes of the warp call it together.
-__device__ void emit_row(const DevPlan &P, const uint8_t *line, const RowRec &r,
-                         const uint32_t *fields, uint8_t *dst, int lane) {
+// Writes a row of cells or values, one thread: a value, or a projection's
+// prefixes and values, as CSV (output.rs:45-81) or JSON; or a whole line as
+// one CSV cell.
+__device__ __forceinline__ void emit_row(const DevPlan &P, const uint8_t *line, const RowRec &r,
+                                         const uint32_t *fields, uint8_t *dst) {
+  uint32_t w = 0;
   if (P.output_kind == 0) {
-    if (!P.csv_mode) {
-      warp_copy(dst, line, r.line_len, lane);
-      if (lane == 0) dst[r.line_len] = '\n';
-    } else if (lane == 0) {
-      uint32_t w = csv_cell_write(dst, line, r.line_len, false, r.row_len - 1);
-      dst[w] = '\n';
-    }
-    return;
-  }
-  uint32_t nf = P.output_kind == 1 ? 1 : P.n_fields;
-  if (P.csv_mode) {
-    if (lane != 0) return;
-    uint32_t w = 0;
-    for (uint32_t f = 0; f < nf; f++) {
-      if (P.output_kind == 2)
-        for (uint32_t k = 0; k < P.prefix_len[f]; k++) dst[w++] = P.blob[P.prefix_off[f] + k];
-      uint32_t off = fields[2 * f], lk = fields[2 * f + 1];
-      uint32_t kind = lk >> 28, esc = (lk >> 27) & 1, len = lk & 0x07FFFFFFu;
-      if (kind == JK_MISSING || kind == JK_NULL) continue;
-      const uint8_t *vp = line + off;
-      if (kind == JK_STR) {
-        uint32_t L = csv_cell_len(vp + 1, len - 2, esc);
-        w += csv_cell_write(dst + w, vp + 1, len - 2, esc, L);
-      } else {
-        uint32_t L = csv_cell_len(vp, len, false);
-        w += csv_cell_write(dst + w, vp, len, false, L);
-      }
-    }
+    w = csv_cell_write(dst, line, r.line_len, false, r.row_len - 1);
     dst[w] = '\n';
     return;
   }
-  // The row as a list of segments (value, or prefix/value pairs then the
-  // suffix, then the newline); lane l writes output bytes l, l+32, ...,
-  // finding each byte's segment with a cursor that only moves forward, and
-  // loads four bytes before storing them.
-  const uint32_t L = r.row_len;
-  uint32_t s = 0, soff = 0, slen;
-  const uint8_t *sp = row_segment(P, line, fields, nf, 0, slen);
-  for (uint32_t base = 0; base < L; base += 128) {
-    uint8_t bb[4];
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint32_t b = base + lane + 32 * k;
-      bb[k] = 0;
-      if (b < L) {
-        while (b >= soff + slen) {
-          soff += slen;
-          sp = row_segment(P, line, fields, nf, ++s, slen);
-        }
-        bb[k] = sp[b - soff];
-      }
+  const bool proj = P.output_kind == 2;
+  const uint32_t nf = proj ? P.n_fields : 1;
+#pragma unroll 1
+  for (uint32_t f = 0; f < nf; f++) {
+    const uint32_t off = fields[2 * f], lk = fields[2 * f + 1];
+    const uint32_t kind = lk >> 28, esc = (lk >> 27) & 1, len = lk & 0x07FFFFFFu;
+    const uint8_t *vp = line + off;
+    if (proj) {
+      const uint32_t n = P.prefix_len[f], at = P.prefix_off[f];
+      for (uint32_t k = 0; k < n; k++) dst[w + k] = P.blob[at + k];
+      w += n;
     }
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint32_t b = base + lane + 32 * k;
-      if (b < L) dst[b] = bb[k];
+    if (!P.csv_mode) {
+      if (kind == JK_MISSING) {
+        dst[w] = 'n';
+        dst[w + 1] = 'u';
+        dst[w + 2] = dst[w + 3] = 'l';
+        w += 4;
+      } else {
+#pragma unroll 4
+        for (uint32_t k = 0; k < len; k++) dst[w + k] = vp[k];
+        w += len;
+      }
+    } else if (kind != JK_MISSING && kind != JK_NULL) {
+      const bool str = kind == JK_STR;
+      const uint8_t *cp = str ? vp + 1 : vp;
+      const uint32_t n = str ? len - 2 : len;
+      w += csv_cell_write(dst + w, cp, n, str && esc, csv_cell_len(cp, n, str && esc));
     }
   }
+  if (proj && !P.csv_mode) {
+    const uint32_t n = P.suffix_len, at = P.suffix_off;
+    for (uint32_t k = 0; k < n; k++) dst[w + k] = P.blob[at + k];
+    w += n;
+  }
+  dst[w] = '\n';
 }
 
 // ---------------------------------------------------------------------------
@@ -1432,12 +1400,15 @@ __global__ void k_batch_finalize(const TileDesc *tiles, const unsigned long long
 // Rows: prefix over the per-tile totals, then emission in line order.
 // ---------------------------------------------------------------------------
 
-// Tiles per block of the rows passes (a multiple of 32, chosen per run by
-// rows_tiles_per_block): small runs take 32 so their row copies still spread
-// over hundreds of blocks, large ones 128 for fewer, fuller blocks.
+// Tiles per block of the rows passes, at most a thread each.  A row costs a
+// few microseconds of dependent loads, whoever copies it, so what counts is
+// how many are in flight: small inputs take 8 tiles a block, up to 262,144
+// tiles 64 (whole lines: 470 us a pass with 64 tiles, 475 with 32, 483 with
+// 128), the largest 128, so the one block that scans the block sums stays
+// short.
 constexpr int kEmitThreads = 128;
 __host__ __device__ inline uint32_t rows_tiles_per_block(unsigned long long n_tiles) {
-  return n_tiles < 148ull * 128 ? 32u : 128u;
+  return n_tiles < 148ull * 8 ? 8u : n_tiles < 262144ull ? 64u : 128u;
 }
 constexpr int kPrefixThreads = 1024;  // the one block that scans the block sums
 
@@ -1478,13 +1449,11 @@ __global__ void __launch_bounds__(kEmitThreads)
   __shared__ unsigned long long s_w[3][kEmitThreads / 32];
   const unsigned long long t0 = (unsigned long long)blockIdx.x * tpb;
   unsigned long long v[3] = {0, 0, 0};
-  for (uint32_t k = threadIdx.x; k < tpb; k += kEmitThreads) {
-    unsigned long long t = t0 + k;
-    if (t < n_tiles) {
-      v[0] += rt[t].rows;
-      v[1] += rt[t].bytes;
-      v[2] += td[t].n_lines;
-    }
+  const unsigned long long t = t0 + threadIdx.x;
+  if (threadIdx.x < tpb && t < n_tiles) {
+    v[0] = rt[t].rows;
+    v[1] = rt[t].bytes;
+    v[2] = td[t].n_lines;
   }
   unsigned long long ex[3], tot[3];
   block_scan3<kEmitThreads>(v, ex, tot, s_w);
@@ -1520,58 +1489,120 @@ __global__ void __launch_bounds__(kPrefixThreads)
   }
 }
 
-// Pass 3: each block takes its `tiles_per_block` tiles kEmitThreads at a time:
-// per-tile prefixes by a block scan, then each warp copies whole tiles'
-// rows, one row at a time, from the input to the output.
-__global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep) {
+// Pass 3: each block takes its `tiles_per_block` tiles: per-tile prefixes by a
+// block scan, then the block's rows, in order.  Whole lines are copied a row a
+// group of lanes.  Rows of values are short, so they take a thread each, which
+// puts its bytes into shared memory; the block then writes the batch's rows,
+// which are contiguous in the output, in whole words.  (768 MB of access-log
+// lines, 6% of them selected: 66 us with a group of lanes a row, 43 so; a warp
+// a row, a tile's rows one after another, took 198.)
+constexpr uint32_t kEmitStage = 8192;  // bytes of a batch of rows kept in shared memory
+
+template <bool kMixed>
+__global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep, const __grid_constant__ DevPlan plan) {
   __shared__ unsigned long long s_w[3][kEmitThreads / 32];
-  __shared__ unsigned long long s_pre[3][kEmitThreads];
-  __shared__ unsigned long long s_rec[kEmitThreads];
-  __shared__ uint32_t s_rows[kEmitThreads];
+  __shared__ unsigned long long s_byte[kEmitThreads], s_line[kEmitThreads], s_rec[kEmitThreads];
+  __shared__ uint32_t s_row[kEmitThreads];  // rows of the block's tiles before this one
+  __shared__ unsigned long long s_span[2];  // output bytes of a batch of rows
+  __shared__ __align__(16) uint8_t s_out[kEmitStage];
   if (ep.ctr->overflow & 3u) return;  // the run is repeated with bigger buffers
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint32_t rec_stride = ep.rec_stride;
-  unsigned long long carry[3];
-  for (int k = 0; k < 3; k++) carry[k] = ep.block_prefix[blockIdx.x * 3 + k];
-  const uint32_t tpb = ep.tiles_per_block;
-  const unsigned long long t0 = (unsigned long long)blockIdx.x * tpb;
-  for (uint32_t sub = 0; sub < tpb; sub += kEmitThreads) {
-    if (t0 + sub >= ep.n_tiles) break;
-    const unsigned long long t = t0 + sub + threadIdx.x;
-    unsigned long long v[3] = {0, 0, 0};
-    unsigned long long rec = 0;
-    if (sub + threadIdx.x < tpb && t < ep.n_tiles) {
-      const RowTile rt = ep.row_tiles[t];
-      v[0] = rt.rows;
-      v[1] = rt.bytes;
-      v[2] = ep.tiles[t].n_lines;
-      rec = rt.rec_begin;
-    }
-    unsigned long long ex[3], tot[3];
-    block_scan3<kEmitThreads>(v, ex, tot, s_w);
-    for (int k = 0; k < 3; k++) s_pre[k][threadIdx.x] = carry[k] + ex[k];
-    s_rec[threadIdx.x] = rec;
-    s_rows[threadIdx.x] = (uint32_t)v[0];
-    __syncthreads();
-    const int n_here = (int)min((uint32_t)kEmitThreads, tpb - sub);
-    for (int i = warp; i < n_here; i += kEmitThreads / 32) {
-      const uint32_t rows = s_rows[i];
-      if (!rows) continue;
-      const DevPlan &P = ep.plans ? ep.plans[ep.in_plan[ep.tile_input[t0 + sub + i]]] : *ep.plan;
-      const unsigned long long row0 = s_pre[0][i], byte0 = s_pre[1][i], line0 = s_pre[2][i];
-      for (uint32_t r = 0; r < rows; r++) {
-        const RowRec *rr = (const RowRec *)(ep.recs + (s_rec[i] + r) * rec_stride);
-        const uint32_t *fl = (const uint32_t *)(rr + 1);
-        const unsigned long long dst_off = byte0 + rr->local_off;
-        emit_row(P, ep.data + rr->line_start, *rr, fl, ep.out + dst_off, lane);
-        if (lane == 0) {
-          ep.row_off[row0 + r] = dst_off;
-          ep.line_idx[row0 + r] = line0 + rr->ordinal;
+  const uint32_t rec_stride = ep.rec_stride, tpb = ep.tiles_per_block;
+  const unsigned long long t0 = (unsigned long long)blockIdx.x * tpb, t = t0 + threadIdx.x;
+  unsigned long long v[3] = {0, 0, 0};
+  unsigned long long rec = 0;
+  if (threadIdx.x < tpb && t < ep.n_tiles) {
+    const RowTile rt = ep.row_tiles[t];
+    v[0] = rt.rows;
+    v[1] = rt.bytes;
+    v[2] = ep.tiles[t].n_lines;
+    rec = rt.rec_begin;
+  }
+  const unsigned long long row0 = ep.block_prefix[blockIdx.x * 3], byte0 = ep.block_prefix[blockIdx.x * 3 + 1],
+                           line0 = ep.block_prefix[blockIdx.x * 3 + 2];
+  unsigned long long ex[3], tot[3];
+  block_scan3<kEmitThreads>(v, ex, tot, s_w);
+  s_row[threadIdx.x] = (uint32_t)ex[0];
+  s_byte[threadIdx.x] = byte0 + ex[1];
+  s_line[threadIdx.x] = line0 + ex[2];
+  s_rec[threadIdx.x] = rec;
+  __syncthreads();
+  const uint32_t rows = (uint32_t)tot[0];
+  // row r's tile: the last with at most r rows before it
+  auto tile_of = [&](uint32_t r) {
+    uint32_t i = 0;
+#pragma unroll
+    for (uint32_t d = kEmitThreads / 2; d; d >>= 1)
+      if (i + d < tpb && s_row[i + d] <= r) i += d;
+    return i;
+  };
+  if (kMixed || (plan.output_kind == 0 && !plan.csv_mode)) {
+    // whole lines; in a mixed batch, rows of any kind
+    const uint32_t g = threadIdx.x % kEmitLanes;
+#pragma unroll 1
+    for (uint32_t r = threadIdx.x / kEmitLanes; r < rows; r += kEmitThreads / kEmitLanes) {
+      const uint32_t i = tile_of(r);
+      const RowRec *rr = (const RowRec *)(ep.recs + (s_rec[i] + (r - s_row[i])) * rec_stride);
+      const RowRec h = *rr;
+      const unsigned long long at = s_byte[i] + h.local_off;
+      const uint8_t *line = ep.data + h.line_start;
+      if (kMixed) {
+        const DevPlan &P = ep.plans[ep.in_plan[ep.tile_input[t0 + i]]];
+        if (P.output_kind != 0 || P.csv_mode) {
+          if (g == 0) {
+            emit_row(P, line, h, (const uint32_t *)(rr + 1), ep.out + at);
+            ep.row_off[row0 + r] = at;
+            ep.line_idx[row0 + r] = s_line[i] + h.ordinal;
+          }
+          continue;
         }
       }
+      group_copy(ep.out + at, line, h.line_len, g);
+      if (g == 0) {
+        ep.out[at + h.line_len] = '\n';
+        ep.row_off[row0 + r] = at;
+        ep.line_idx[row0 + r] = s_line[i] + h.ordinal;
+      }
     }
-    for (int k = 0; k < 3; k++) carry[k] += tot[k];
+    return;
+  }
+  if constexpr (!kMixed)
+#pragma unroll 1
+  for (uint32_t r0 = 0; r0 < rows; r0 += kEmitThreads) {
+    const uint32_t r = r0 + threadIdx.x;
+    RowRec h;
+    const uint32_t *fl = nullptr;
+    unsigned long long at = 0;
+    if (r < rows) {
+      const uint32_t i = tile_of(r);
+      const RowRec *rr = (const RowRec *)(ep.recs + (s_rec[i] + (r - s_row[i])) * rec_stride);
+      h = *rr;
+      fl = (const uint32_t *)(rr + 1);
+      at = s_byte[i] + h.local_off;
+      ep.row_off[row0 + r] = at;
+      ep.line_idx[row0 + r] = s_line[i] + h.ordinal;
+      if (threadIdx.x == 0) s_span[0] = at;
+      if (r + 1 == rows || threadIdx.x == kEmitThreads - 1) s_span[1] = at + h.row_len;
+    }
     __syncthreads();
+    // the batch's place in the output and, from the word it starts in, in s_out
+    const unsigned long long b0 = s_span[0], b1 = s_span[1];
+    const uint32_t lead = (uint32_t)((uintptr_t)(ep.out + b0) & 3u);
+    const bool staged = b1 - b0 + 4 <= kEmitStage;
+    if (r < rows)
+      emit_row(plan, ep.data + h.line_start, h, fl, staged ? s_out + lead + (uint32_t)(at - b0) : ep.out + at);
+    __syncthreads();
+    if (staged) {
+      uint8_t *const w0 = ep.out + b0 - lead;  // a word boundary
+      const uint32_t end = lead + (uint32_t)(b1 - b0);
+      for (uint32_t k = 4 * threadIdx.x; k < end; k += 4 * kEmitThreads) {
+        if (k >= lead && k + 4 <= end) {
+          *(uint32_t *)(w0 + k) = *(const uint32_t *)(s_out + k);
+        } else {
+          for (uint32_t j = max(k, lead); j < min(k + 4, end); j++) w0[j] = s_out[j];
+        }
+      }
+      __syncthreads();
+    }
   }
 }
 
