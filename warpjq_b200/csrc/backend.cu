@@ -102,6 +102,8 @@ struct RunBufs {
   DevBuf<unsigned long long> g_slots;
   DevBuf<GroupKeyDesc> g_keys;
   DevBuf<GroupAcc> g_acc;
+  DevBuf<warpjq_group_ext> g_ext;  // the compacted results, and each one's batch input
+  DevBuf<uint32_t> g_in;
 
   // current capacities
   unsigned long long rec_cap_per_cta = 0;
@@ -124,14 +126,13 @@ struct RunBufs {
     b_rec_cursor.release();
     recs.release(); out.release(); row_off.release(); line_idx.release();
     block_lines.release(); deep.release(); tmpl.release(); g_slots.release();
-    g_keys.release(); g_acc.release();
+    g_keys.release(); g_acc.release(); g_ext.release(); g_in.release();
   }
 };
 
 constexpr unsigned kReduceBlocks = 256;
 
-__global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, uint32_t key_cap, TemplateBuf *tmpl,
-                            uint32_t n_tmpl) {
+__global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, TemplateBuf *tmpl, uint32_t n_tmpl) {
   unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
   unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
   if (tid == 0) {
@@ -147,7 +148,6 @@ __global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, uint
   for (unsigned long long i = tid; i < n_tmpl; i += stride) tmpl[i].state = tmpl[i].tries = 0;
   if (g.slots) {
     for (unsigned long long i = tid; i < g_cap; i += stride) g.slots[i] = 0;
-    for (unsigned long long i = tid; i < key_cap; i += stride) group_acc_init(g.acc[i]);
   }
 }
 
@@ -175,6 +175,12 @@ struct Slot {
   size_t h_rows_cap = 0;
   warpjq_group *h_groups = nullptr;
   size_t h_groups_cap = 0;
+  // group results copied from the device: page-locked up to kPinnedGroups
+  warpjq_group_ext *h_ext = nullptr;
+  uint32_t *h_in = nullptr;
+  size_t h_ext_cap = 0;
+  std::vector<warpjq_group_ext> v_ext;
+  std::vector<uint32_t> v_in;
   bool launched = false;
   uint32_t kernels = 0;
   // page-locked staging of a batch's tables (copied from here without a
@@ -205,7 +211,6 @@ struct warpjq_ctx {
   const uint8_t *dev_data = nullptr;
   unsigned long long dev_n = 0;
   cudaStream_t dev_stream = nullptr;
-  std::vector<warpjq_group_ext> dev_groups;
   // batched runs (warpjq_batch_launch): host copies of the tables
   struct Batch {
     bool active = false;
@@ -308,6 +313,8 @@ warpjq_status ensure_bufs(warpjq_ctx *c, Slot &s, unsigned long long n,
     CK(rb.g_slots.ensure(rb.g_cap, st, cap), "alloc group table");
     CK(rb.g_keys.ensure(rb.g_key_cap, st, cap), "alloc group keys");
     CK(rb.g_acc.ensure(rb.g_key_cap, st, cap), "alloc group accumulators");
+    CK(rb.g_ext.ensure(rb.g_key_cap, st, cap), "alloc group results");
+    CK(rb.g_in.ensure(rb.g_key_cap, st, cap), "alloc group results");
   }
   return WARPJQ_OK;
 }
@@ -434,7 +441,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
   GroupTable g = group_view(rb, groups);
   const uint32_t n_tmpl = b && b->mixed ? (uint32_t)b->plans.size() : 1u;
   CK(rb.tmpl.ensure(n_tmpl, st, capturing), "alloc line templates");
-  k_reset_run<<<256, 256, 0, st>>>(rb.ctr.p, g, groups ? rb.g_cap : 0, groups ? rb.g_key_cap : 0, rb.tmpl.p, n_tmpl);
+  k_reset_run<<<256, 256, 0, st>>>(rb.ctr.p, g, groups ? rb.g_cap : 0, rb.tmpl.p, n_tmpl);
   s.kernels++;
   CK(cudaGetLastError(), "launch reset");
   if (n > 0 && n_tiles > 0) {
@@ -549,6 +556,11 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
       s.kernels += 3;
       CK(cudaGetLastError(), "launch rows");
     }
+    if (groups) {
+      k_groups_compact<<<(unsigned)std::min<uint32_t>((rb.g_key_cap + 255) / 256, 4u * c->num_sms), 256, 0, st>>>(
+          rb.ctr.p, rb.g_keys.p, rb.g_acc.p, rb.g_key_cap, rb.g_ext.p, rb.g_in.p);
+      s.kernels++;
+    }
     k_reduce_tiles<<<kReduceBlocks, kReduceThreads, 0, st>>>(n_tiles, rb.tiles.p, rb.ctr.p,
                                                              rb.block_lines.p);
     s.kernels++;
@@ -598,6 +610,8 @@ bool grow_after_overflow(warpjq_ctx *c, Slot &s, const RunCounters &h, unsigned 
     rb.g_slots.release();
     rb.g_keys.release();
     rb.g_acc.release();
+    rb.g_ext.release();
+    rb.g_in.release();
     again = true;
   }
   if (h.overflow & 8u) {  // deep nesting
@@ -606,6 +620,23 @@ bool grow_after_overflow(warpjq_ctx *c, Slot &s, const RunCounters &h, unsigned 
     again = true;
   }
   return again;
+}
+
+constexpr size_t kFirstGroups = 64;          // copied with the counters
+constexpr size_t kPinnedGroups = 1u << 20;  // page-locked room for results grows up to this (92 MB)
+
+warpjq_status ensure_host_groups(Slot &s, size_t n, char *err, size_t err_len) {
+  if (n <= s.h_ext_cap) return WARPJQ_OK;
+  if (s.h_ext) cudaFreeHost(s.h_ext);
+  if (s.h_in) cudaFreeHost(s.h_in);
+  s.h_ext = nullptr;
+  s.h_in = nullptr;
+  s.h_ext_cap = 0;
+  const size_t cap = std::max(n, std::min(n + n / 4, kPinnedGroups));
+  CK(cudaHostAlloc((void **)&s.h_ext, cap * sizeof(warpjq_group_ext), cudaHostAllocDefault), "pinned groups");
+  CK(cudaHostAlloc((void **)&s.h_in, cap * sizeof(uint32_t), cudaHostAllocDefault), "pinned groups");
+  s.h_ext_cap = cap;
+  return WARPJQ_OK;
 }
 
 // Runs synchronously until the result is complete; leaves counters in h.
@@ -618,9 +649,17 @@ warpjq_status run_to_completion(warpjq_ctx *c, Slot &s, const uint8_t *d_data,
       warpjq_status rc = enqueue_run(c, s, d_data, n, st, err, err_len, b);
       if (rc != WARPJQ_OK) return rc;
     }
-    CK(cudaMemcpyAsync(&h, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st),
+    CK(cudaMemcpyAsync(s.h_ctr, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st),
        "D2H counters");
+    if (run_grouped(c, b)) {  // few groups come along, without a second wait
+      warpjq_status rc = ensure_host_groups(s, kFirstGroups, err, err_len);
+      if (rc != WARPJQ_OK) return rc;
+      CK(cudaMemcpyAsync(s.h_ext, s.rb.g_ext.p, kFirstGroups * sizeof(warpjq_group_ext), cudaMemcpyDeviceToHost, st),
+         "D2H groups");
+      if (b) CK(cudaMemcpyAsync(s.h_in, s.rb.g_in.p, kFirstGroups * 4, cudaMemcpyDeviceToHost, st), "D2H groups");
+    }
     CK(cudaStreamSynchronize(st), "stream sync");
+    h = *s.h_ctr;
     if (h.error) {
       set_err(err, err_len, "the scan kernel raised its error flag");
       return WARPJQ_ERR_CUDA;
@@ -661,6 +700,7 @@ uint64_t bufs_signature(const warpjq_ctx *c) {
   mix((uintptr_t)rb.deep.p); mix(rb.deep.n);
   mix((uintptr_t)rb.tmpl.p); mix(rb.tmpl.n);
   mix((uintptr_t)rb.g_slots.p); mix((uintptr_t)rb.g_keys.p); mix((uintptr_t)rb.g_acc.p);
+  mix((uintptr_t)rb.g_ext.p); mix((uintptr_t)rb.g_in.p);
   mix(rb.rec_cap_per_cta); mix(rb.out_cap); mix(rb.rows_cap); mix(rb.g_cap); mix(rb.g_key_cap);
   mix(rb.deep_levels); mix(c->tile_bytes); mix(c->halo_bytes); mix(c->grid); mix(c->scan_smem);
   return h;
@@ -774,6 +814,8 @@ static void free_slot(Slot &s) {
   if (s.h_line64) cudaFreeHost(s.h_line64);
   if (s.h_line32) cudaFreeHost(s.h_line32);
   if (s.h_groups) cudaFreeHost(s.h_groups);
+  if (s.h_ext) cudaFreeHost(s.h_ext);
+  if (s.h_in) cudaFreeHost(s.h_in);
   if (s.scan_t0) cudaEventDestroy(s.scan_t0);
   if (s.scan_t1) cudaEventDestroy(s.scan_t1);
   if (s.h_btab) cudaFreeHost(s.h_btab);
@@ -886,42 +928,32 @@ static warpjq_status ensure_pinned(Slot &s, size_t out_bytes, size_t rows, size_
   return WARPJQ_OK;
 }
 
-// Copies the compacted group table of a finished run to the host.
-static warpjq_status fetch_groups(warpjq_ctx *ctx, Slot &s, const RunCounters &h,
-                                  std::vector<warpjq_group_ext> &out, char *err, size_t err_len,
-                                  std::vector<uint32_t> *inputs = nullptr) {
-  out.clear();
-  if (inputs) inputs->clear();
-  uint32_t nk = std::min<uint32_t>(h.n_keys, s.rb.g_key_cap);
-  if (!nk) return WARPJQ_OK;
-  std::vector<GroupKeyDesc> keys(nk);
-  std::vector<GroupAcc> acc(nk);
-  RunBufs &rb = s.rb;
-  CK(cudaMemcpy(keys.data(), rb.g_keys.p, nk * sizeof(GroupKeyDesc), cudaMemcpyDeviceToHost),
-     "D2H group keys");
-  CK(cudaMemcpy(acc.data(), rb.g_acc.p, nk * sizeof(GroupAcc), cudaMemcpyDeviceToHost),
-     "D2H group accumulators");
-  for (uint32_t k = 0; k < nk; k++) {
-    const GroupAcc &a = acc[k];
-    if (a.count == 0) continue;  // an id allocated by a racing insert that lost
-    warpjq_group_ext g{};
-    g.key_off = keys[k].off;
-    g.key_len = keys[k].len;
-    g.key_kind = keys[k].kind;
-    g.count = a.count;
-    g.numeric = a.numeric;
-    g.isum_lo = a.isum_lo;
-    g.isum_hi = a.isum_hi;
-    g.n_int = a.n_int;
-    // exact sums, rounded once (fixsum.cuh)
-    g.fsum = fix_to_double(a.fix, 0, 0) + a.fbig;
-    g.min = a.numeric ? min_of_bits(a.min_bits) : __builtin_huge_val();
-    g.max = a.numeric ? max_of_bits(a.max_bits) : -__builtin_huge_val();
-    g.sum = fix_to_double(a.fix, a.isum_lo, a.isum_hi) + a.fbig;
-    out.push_back(g);
-    if (inputs) inputs->push_back(keys[k].input);
+// The group results of a finished run: `n` of them at `gs`, and their batch
+// inputs at `gin` (with `inputs`), valid until the slot's next run.
+static warpjq_status fetch_groups(Slot &s, const RunCounters &h, cudaStream_t st, bool inputs,
+                                  const warpjq_group_ext *&gs, const uint32_t *&gin, size_t &n, char *err,
+                                  size_t err_len) {
+  n = h.n_groups;
+  warpjq_group_ext *ext = s.h_ext;
+  uint32_t *in = s.h_in;
+  if (n > kFirstGroups) {
+    if (n > kPinnedGroups) {
+      s.v_ext.resize(n);
+      s.v_in.resize(inputs ? n : 0);
+      ext = s.v_ext.data();
+      in = s.v_in.data();
+    } else {
+      warpjq_status rc = ensure_host_groups(s, n, err, err_len);
+      if (rc != WARPJQ_OK) return rc;
+      ext = s.h_ext;
+      in = s.h_in;
+    }
+    CK(cudaMemcpyAsync(ext, s.rb.g_ext.p, n * sizeof(warpjq_group_ext), cudaMemcpyDeviceToHost, st), "D2H groups");
+    if (inputs) CK(cudaMemcpyAsync(in, s.rb.g_in.p, n * 4, cudaMemcpyDeviceToHost, st), "D2H groups");
+    CK(cudaStreamSynchronize(st), "stream sync");
   }
-  (void)ctx;
+  gs = ext;
+  gin = in;
   return WARPJQ_OK;
 }
 
@@ -954,12 +986,14 @@ warpjq_status warpjq_wait(warpjq_ctx *ctx, uint32_t slot, warpjq_chunk_result *o
       out->agg.max = h.agg_numeric ? max_of_bits(h.agg_max_bits) : -__builtin_huge_val();
       out->agg.saw_non_numeric = h.agg_saw_non_numeric;
     } else {
-      std::vector<warpjq_group_ext> gs;
-      rc = fetch_groups(ctx, s, h, gs, err, err_len);
+      const warpjq_group_ext *gs;
+      const uint32_t *gin;
+      size_t n;
+      rc = fetch_groups(s, h, s.stream, false, gs, gin, n, err, err_len);
       if (rc != WARPJQ_OK) return rc;
-      rc = ensure_pinned(s, 0, 0, gs.size(), err, err_len);
+      rc = ensure_pinned(s, 0, 0, n, err, err_len);
       if (rc != WARPJQ_OK) return rc;
-      for (size_t k = 0; k < gs.size(); k++) {
+      for (size_t k = 0; k < n; k++) {
         warpjq_group &d = s.h_groups[k];
         d.key_off = (uint32_t)gs[k].key_off;
         d.key_len = gs[k].key_len;
@@ -972,7 +1006,7 @@ warpjq_status warpjq_wait(warpjq_ctx *ctx, uint32_t slot, warpjq_chunk_result *o
         d.max = gs[k].max;
       }
       out->groups = s.h_groups;
-      out->n_groups = (uint32_t)gs.size();
+      out->n_groups = (uint32_t)n;
     }
     return WARPJQ_OK;
   }
@@ -1032,6 +1066,8 @@ warpjq_status warpjq_set_group_capacity(warpjq_ctx *ctx, uint32_t keys) {
     rb.g_slots.release();
     rb.g_keys.release();
     rb.g_acc.release();
+    rb.g_ext.release();
+    rb.g_in.release();
     rb.g_cap = rb.g_key_cap = 0;
   };
   for (auto &s : ctx->slots) drop(s.rb);
@@ -1134,10 +1170,11 @@ warpjq_status warpjq_collect_device(warpjq_ctx *ctx, warpjq_device_result *out, 
   out->sum = h.sum_total;
   out->saw_non_numeric = h.agg_saw_non_numeric;
   if (P.output_kind == WARPJQ_OUT_AGG && P.group_slot >= 0) {
-    rc = fetch_groups(ctx, s, h, ctx->dev_groups, err, err_len);
+    const uint32_t *gin;
+    size_t n;
+    rc = fetch_groups(s, h, ctx->dev_stream, false, out->groups, gin, n, err, err_len);
     if (rc != WARPJQ_OK) return rc;
-    out->groups = ctx->dev_groups.data();
-    out->n_groups = (uint32_t)ctx->dev_groups.size();
+    out->n_groups = (uint32_t)n;
   }
   out->kernels_launched = s.kernels;
   out->scan_ms = 0.0;
@@ -1271,15 +1308,16 @@ warpjq_status warpjq_batch_collect(warpjq_ctx *ctx, warpjq_batch_item *items,
   // Groups ordered by input (stable within an input).
   std::vector<uint32_t> first(n + 1, 0);
   if (grouped) {
-    std::vector<warpjq_group_ext> gs;
-    std::vector<uint32_t> gin;
-    rc = fetch_groups(ctx, s, h, gs, err, err_len, &gin);
+    const warpjq_group_ext *gs;
+    const uint32_t *gin;
+    size_t ng;
+    rc = fetch_groups(s, h, b.stream, true, gs, gin, ng, err, err_len);
     if (rc != WARPJQ_OK) return rc;
-    for (uint32_t in : gin) first[in + 1]++;
+    for (size_t k = 0; k < ng; k++) first[gin[k] + 1]++;
     for (uint32_t i = 0; i < n; i++) first[i + 1] += first[i];
-    b.groups.assign(gs.size(), warpjq_group_ext{});
+    b.groups.resize(ng);
     std::vector<uint32_t> fill(first.begin(), first.end() - 1);
-    for (size_t k = 0; k < gs.size(); k++) b.groups[fill[gin[k]]++] = gs[k];
+    for (size_t k = 0; k < ng; k++) b.groups[fill[gin[k]]++] = gs[k];
   } else {
     b.groups.clear();
   }
