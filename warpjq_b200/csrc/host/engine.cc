@@ -23,6 +23,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -355,6 +356,8 @@ struct Writer {
       buf += '\n';
     }
   }
+  void device_groups(const std::string &name, uint32_t kind, const uint8_t *data, const warpjq_group_ext *gs,
+                     uint32_t n);
   // Hands the output to the caller as one malloc'd, NUL-terminated buffer.
   char *finish(size_t &len) {
     if (fmt == WARPJQ_FMT_COUNT) buf = std::to_string(rows) + "\n";
@@ -374,6 +377,153 @@ struct Writer {
     return o;
   }
 };
+
+// A device group on its way to the output: its key's place in the output
+// order (GroupKey's), and where its entry is.
+struct GroupRow {
+  uint64_t pre;      // number: its order bits; else the first 8 bytes, big-endian
+  const uint8_t *p;  // the key's bytes (a string's decoded, any other's text)
+  uint32_t len, at;
+  uint8_t rank;
+  bool operator<(const GroupRow &o) const {
+    if (rank != o.rank) return rank < o.rank;
+    if (pre != o.pre) return pre < o.pre;
+    const int c = memcmp(p, o.p, std::min(len, o.len));
+    return c ? c < 0 : len < o.len;
+  }
+};
+
+// f(0) .. f(n - 1), each on a thread of its own (the last on this one).
+template <class F>
+void on_threads(unsigned n, F &&f) {
+  std::vector<std::thread> ws;
+  for (unsigned t = 0; t + 1 < n; t++) {
+    try {
+      ws.emplace_back(f, t);
+    } catch (const std::system_error &) {  // no thread to be had
+      f(t);
+    }
+  }
+  f(n - 1);
+  for (auto &w : ws) w.join();
+}
+
+// The groups of a device-resident result in output order.  From 16,384 groups
+// on the work is split over up to 16 threads (reading the keys, all over the
+// input; splitting them into ranges of the output order by a sample; sorting
+// and printing each range): 150,000 groups took 54 ms as one sort of
+// key strings, 3 ms so; below, threads cost more than they save.
+void Writer::device_groups(const std::string &name, uint32_t kind, const uint8_t *data, const warpjq_group_ext *gs,
+                           uint32_t n) {
+  rows += n;
+  if (fmt == WARPJQ_FMT_COUNT || !n) return;
+  const unsigned T = n < 16384 ? 1u : std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+  auto part = [&](unsigned t) { return (uint32_t)((uint64_t)n * t / T); };
+  std::vector<GroupRow> in(n), out(T > 1 ? n : 0);
+  std::vector<std::vector<std::unique_ptr<std::string>>> decoded(T);  // keys with escapes
+  on_threads(T, [&](unsigned t) {
+    for (uint32_t k = part(t); k < part(t + 1); k++) {
+      const warpjq_group_ext &g = gs[k];
+      GroupRow r{0, data + g.key_off, g.key_len, k, 0};
+      switch (g.key_kind) {
+        case 0: case 1: r.len = 0; break;
+        case 2: r.rank = (r.len == 4 && memcmp(r.p, "true", 4) == 0) ? 2 : 1; break;
+        case 3: r.rank = 3; break;
+        case 4:
+          r.rank = 4;
+          if (memchr(r.p, '\\', r.len)) {
+            decoded[t].emplace_back(new std::string(unescape(r.p, r.len)));
+            r.p = (const uint8_t *)decoded[t].back()->data();
+            r.len = (uint32_t)decoded[t].back()->size();
+          }
+          break;
+        default: r.rank = 5;
+      }
+      if (r.rank == 3) {
+        r.pre = order_bits(strtod(std::string((const char *)r.p, r.len).c_str(), nullptr));
+      } else {
+        for (uint32_t j = 0; j < 8; j++) r.pre = r.pre << 8 | (j < r.len ? r.p[j] : 0u);
+      }
+      in[k] = r;
+    }
+  });
+  // ranges of the output order: range t's rows are out[begin[t], begin[t + 1])
+  std::vector<uint32_t> begin(T + 1, 0);
+  if (T > 1) {
+    std::vector<GroupRow> sample;
+    for (uint32_t k = 0; k < 32 * T; k++) sample.push_back(in[(uint64_t)n * k / (32 * T)]);
+    std::sort(sample.begin(), sample.end());
+    std::vector<GroupRow> cut;
+    for (unsigned t = 1; t < T; t++) cut.push_back(sample[32 * t]);
+    auto range = [&](const GroupRow &r) { return (unsigned)(std::upper_bound(cut.begin(), cut.end(), r) - cut.begin()); };
+    std::vector<std::vector<uint32_t>> count(T, std::vector<uint32_t>(T, 0));
+    on_threads(T, [&](unsigned t) {
+      for (uint32_t k = part(t); k < part(t + 1); k++) count[t][range(in[k])]++;
+    });
+    uint32_t run = 0;
+    for (unsigned r = 0; r < T; r++) {
+      begin[r] = run;
+      for (unsigned t = 0; t < T; t++) {
+        const uint32_t c = count[t][r];
+        count[t][r] = run;
+        run += c;
+      }
+    }
+    on_threads(T, [&](unsigned t) {
+      for (uint32_t k = part(t); k < part(t + 1); k++) out[count[t][range(in[k])]++] = in[k];
+    });
+  } else {
+    out.swap(in);
+  }
+  begin[T] = n;
+  std::string head = "{", mid = ",";
+  json_string(head, (const uint8_t *)name.data(), name.size());
+  head += ':';
+  const char *an = agg_name(kind);
+  json_string(mid, (const uint8_t *)an, strlen(an));
+  mid += ':';
+  std::vector<std::string> text(T);
+  on_threads(T, [&](unsigned t) {
+    std::sort(out.begin() + begin[t], out.begin() + begin[t + 1]);
+    std::string o;
+    o.reserve((size_t)(begin[t + 1] - begin[t]) * 48);
+    for (uint32_t k = begin[t]; k < begin[t + 1]; k++) {
+      const GroupRow &r = out[k];
+      const warpjq_group_ext &g = gs[r.at];
+      Agg a;
+      a.merge(g.count, g.numeric, g.sum, g.min, g.max);
+      double v;
+      const std::string val = a.finish(kind, v) ? format_number(v) : "null";
+      const char *fixed = r.rank == 0 ? "null" : r.rank == 1 ? "false" : r.rank == 2 ? "true" : nullptr;
+      if (fmt == WARPJQ_FMT_CSV) {
+        if (fixed) o += fixed;
+        else csv_cell(o, r.p, r.len);
+        o += ',';
+        o += val;
+      } else {
+        o += head;
+        if (fixed) o += fixed;
+        else if (r.rank == 4) json_string(o, r.p, r.len);
+        else o.append((const char *)r.p, r.len);
+        o += mid;
+        o += val;
+        o += '}';
+      }
+      o += '\n';
+    }
+    text[t] = std::move(o);
+  });
+  if (T == 1) {
+    buf += text[0];
+    return;
+  }
+  oom |= !bulk_rows.append(buf.data(), buf.size());
+  buf.clear();
+  size_t total = bulk_rows.n;
+  for (auto &x : text) total += x.size();
+  oom |= !bulk_rows.reserve(total + 1);
+  for (auto &x : text) oom |= !bulk_rows.append(x.data(), x.size());
+}
 
 }  // namespace wjqh
 
@@ -1126,16 +1276,7 @@ static void render_head(const warpjq_query *q, Writer &w, uint64_t count, uint64
       a.merge(count, numeric, sum, mn, mx);
       w.aggregate(P.agg, a);
     } else {
-      std::vector<std::pair<GroupKey, Agg>> gs;
-      gs.reserve(n_groups);
-      for (uint32_t k = 0; k < n_groups; k++) {
-        const warpjq_group_ext &g = groups[k];
-        Agg a;
-        a.merge(g.count, g.numeric, g.sum, g.min, g.max);
-        gs.push_back({device_key(data, g.key_off, g.key_len, g.key_kind), a});
-      }
-      std::sort(gs.begin(), gs.end(), [](const auto &a, const auto &b) { return a.first < b.first; });
-      w.groups(P.group_key_name(), P.agg, gs);
+      w.device_groups(P.group_key_name(), P.agg, data, groups, n_groups);
     }
   } else {
     w.rows = n_selected;
