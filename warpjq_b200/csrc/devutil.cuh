@@ -240,36 +240,6 @@ __device__ inline int cmp_str_body(const uint8_t *body, uint32_t n, bool has_esc
   }
 }
 
-// FNV-1a over the decoded bytes of a string body.
-__device__ inline uint32_t hash_str_body(const uint8_t *body, uint32_t n, bool has_escape) {
-  uint32_t h = 0x811c9dc5u;
-  if (!has_escape) {
-#pragma unroll 1
-    for (uint32_t k = 0; k < n; k++) {
-      h ^= body[k];
-      h *= 0x01000193u;
-    }
-    return h;
-  }
-  StrDecoder d(body, n);
-#pragma unroll 1
-  for (int c; (c = d.next()) >= 0;) {
-    h ^= (uint32_t)c;
-    h *= 0x01000193u;
-  }
-  return h;
-}
-
-__device__ inline uint32_t hash_raw(const uint8_t *p, uint32_t n) {
-  uint32_t h = 0x811c9dc5u;
-#pragma unroll 1
-  for (uint32_t k = 0; k < n; k++) {
-    h ^= p[k];
-    h *= 0x01000193u;
-  }
-  return h;
-}
-
 // ---------------------------------------------------------------------------
 // Number parsing.
 //

@@ -24,6 +24,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/warpjq_ext.h"
@@ -48,8 +49,6 @@ constexpr int kReduceThreads = 128;          // block size of the per-tile reduc
 constexpr int kScanBlocksPerSM = 20;
 constexpr int kScanBlocksPerSMRows = 20;
 constexpr int kScanBlocksPerSMGrouped = 16;
-
-constexpr int kGroupCache = 16;  // per-CTA group accumulators kept in shared memory
 
 // A CTA's line counts and ungrouped aggregate, in shared memory: each round
 // of up to 32 lines is reduced in the warp (ballots, warp reductions) and
@@ -158,16 +157,37 @@ struct GroupKeyDesc {
 };
 static_assert(sizeof(GroupKeyDesc) == 24, "group key descriptor");
 
-// A CTA's private accumulators for up to kGroupCache keys (direct-mapped by
-// key id), merged into the global records when the CTA finishes.  Hot keys
-// then cost shared-memory atomics instead of contended global ones.
-struct GroupCache {
-  uint32_t tag[kGroupCache];  // key id held by the entry, or 0xFFFFFFFF
-  GroupAcc acc[kGroupCache];
+// A CTA's own record of the first 32 short keys it meets, by their hash (the
+// place it names, or the next free one) and bytes, with their accumulators: a key that
+// comes again costs no probe of the table in global memory (a slot, the key's
+// descriptor and its bytes, one after another) and no global atomics, where
+// the hot keys of all CTAs would meet.  Sums and averages keep 16 keys with
+// whole accumulators, the others 32 with their first halves.  Entries hold
+// keys of one input; a batch's next input starts over.
+//
+// Most rounds are counts, extremes and sums of plain integers: those go by
+// 32-bit shared atomics into n, num, lo and hi (a sum's values as two halves;
+// for extremes, lo counts the integers), which hold kFoldLines lines before
+// they are folded into the accumulators.
+constexpr uint32_t kKeyCache = 32;       // one lane clears one
+constexpr uint32_t kKeyCacheBytes = 24;  // longest key kept
+constexpr uint32_t kKeyAccBytes = 2048;
+constexpr uint32_t kFoldLines = 32768;   // 65,535 of them could overflow lo
+struct KeyCache {
+  uint32_t hash[kKeyCache];  // 0: free
+  uint32_t meta[kKeyCache];  // length | kind << 24
+  uint32_t kid[kKeyCache];
+  uint32_t bytes[kKeyCache][kKeyCacheBytes / 4];  // zero past the key's end
+  uint32_t n[kKeyCache], num[kKeyCache], lo[kKeyCache], hi[kKeyCache];
+  unsigned long long acc[kKeyAccBytes / 8];
+  __device__ __forceinline__ GroupAcc &at(uint32_t e, bool whole) {
+    return *(GroupAcc *)((uint8_t *)acc + e * (whole ? 128u : 64u));
+  }
 };
+static_assert(offsetof(GroupAcc, fix) == 64, "the first half is all but the limbs");
 
 __host__ __device__ inline size_t scan_smem_bytes(uint32_t T, uint32_t H, bool groups) {
-  return scan_smem_base(T, H) + (groups ? sizeof(GroupCache) : 0);
+  return scan_smem_base(T, H) + (groups ? sizeof(KeyCache) : 0);
 }
 
 struct GroupTable {
@@ -295,9 +315,128 @@ __device__ __forceinline__ bool key_bytes_equal(const KeyRef &a, const uint8_t *
   }
 }
 
+// The hash of a key's (decoded) bytes, four at a time, zero past the end.
+struct KeyHasher {
+  uint32_t h = 0x811C9DC5u;
+  __device__ __forceinline__ void word(uint32_t w) {
+    h = (h ^ w) * 0x9E3779B1u;
+    h ^= h >> 15;
+  }
+  __device__ __forceinline__ uint32_t done(uint32_t len, uint32_t kind, uint32_t input) {
+    h ^= len * 0x85EBCA6Bu ^ kind * 0xC2B2AE35u ^ input * 0x27D4EB2Fu;
+    h = (h ^ (h >> 16)) * 0x7FEB352Du;
+    h ^= h >> 15;
+    return h ? h : 1u;
+  }
+};
+
+// The mask of the bytes of a key's word k (of a key of len bytes).
+__device__ __forceinline__ uint32_t key_word_mask(uint32_t len, uint32_t k) {
+  return 4 * k + 4 <= len ? 0xFFFFFFFFu : 0xFFFFFFFFu >> (8 * (4 * k + 4 - len));
+}
+
+// The bytes of a key of up to kKeyCacheBytes at w[off, off + len) of a window,
+// zero past its end.
+__device__ __forceinline__ void key_words(const uint8_t *w, uint32_t off, uint32_t len,
+                                          uint32_t kw[kKeyCacheBytes / 4]) {
+  const uint32_t *q = (const uint32_t *)w + (off >> 2);
+  const uint32_t sh = (off & 3u) * 8u;
+  uint32_t lo = q[0];
+#pragma unroll
+  for (uint32_t k = 0; k < kKeyCacheBytes / 4; k++) {
+    const uint32_t hi = q[k + 1];
+    kw[k] = 4 * k < len ? __funnelshift_r(lo, hi, sh) & key_word_mask(len, k) : 0u;
+    lo = hi;
+  }
+}
+
+// kcache without keys.
+__device__ __noinline__ void keys_clear(KeyCache &c, bool whole, int lane) {
+  __syncwarp();
+  c.hash[lane] = c.n[lane] = c.num[lane] = c.lo[lane] = c.hi[lane] = 0;
+  if (whole) {
+    if (lane < (int)kKeyCache / 2) group_acc_init(c.at(lane, true));
+  } else {
+    GroupAcc &a = c.at(lane, false);
+    a.count = a.numeric = a.isum_lo = a.isum_hi = a.n_int = 0;
+    a.min_bits = ~0ull;
+    a.max_bits = 0;
+    a.fbig = 0.0;
+  }
+  __syncwarp();
+}
+
+// The 32-bit sums into the accumulators they belong to.
+__device__ __noinline__ void keys_fold(KeyCache &c, bool whole, int lane) {
+  __syncwarp();
+  if (c.n[lane]) {
+    GroupAcc &a = c.at(lane, whole);
+    a.count += c.n[lane];
+    a.numeric += c.num[lane];
+    a.n_int += whole ? c.num[lane] : c.lo[lane];
+    if (whole) {
+      const unsigned long long x = c.lo[lane] + ((unsigned long long)c.hi[lane] << 16), lo = a.isum_lo + x;
+      a.isum_hi += lo < x ? 1ull : 0ull;
+      a.isum_lo = lo;
+    }
+    c.n[lane] = c.num[lane] = c.lo[lane] = c.hi[lane] = 0;
+  }
+  __syncwarp();
+}
+
+// Adds kcache's accumulators to the keys' global records.
+__device__ __noinline__ void keys_flush(KeyCache &c, const GroupTable &g, bool whole, int lane) {
+  keys_fold(c, whole, lane);
+  if (lane >= (int)(whole ? kKeyCache / 2 : kKeyCache) || !c.hash[lane]) return;
+  const GroupAcc &x = c.at(lane, whole);
+  GroupAcc &a = g.acc[c.kid[lane]];
+  if (x.count) atomicAdd(&a.count, x.count);
+  if (x.numeric) {
+    atomicAdd(&a.numeric, x.numeric);
+    atomicMin(&a.min_bits, x.min_bits);
+    atomicMax(&a.max_bits, x.max_bits);
+  }
+  if (x.n_int) {
+    const unsigned long long old = atomicAdd(&a.isum_lo, x.isum_lo);
+    const unsigned long long carry = (old + x.isum_lo) < old ? 1ull : 0ull;
+    if (x.isum_hi + carry) atomicAdd(&a.isum_hi, x.isum_hi + carry);
+    atomicAdd(&a.n_int, x.n_int);
+  }
+  if (whole) {  // whatever numeric says: a line that led the key's round may have counted in the global record
+#pragma unroll 1
+    for (int d = 0; d < kFixDigits; d++)
+      if (x.fix[d]) atomicAdd((unsigned long long *)&a.fix[d], (unsigned long long)x.fix[d]);
+    if (x.fbig != 0.0) atomicAdd(&a.fbig, x.fbig);
+  }
+}
+
+// Any key, byte by byte: the same hash for the same decoded bytes.
+__device__ __noinline__ uint32_t hash_key_far(const uint8_t *p, uint32_t len, bool esc, uint32_t kind,
+                                              uint32_t input) {
+  KeyHasher x;
+  uint32_t w = 0, n = 0;
+  auto put = [&](uint32_t c) {
+    w |= c << (8 * (n & 3u));
+    if ((++n & 3u) == 0) {
+      x.word(w);
+      w = 0;
+    }
+  };
+  if (esc) {
+    StrDecoder d(p, len);
+#pragma unroll 1
+    for (int c; (c = d.next()) >= 0;) put((uint32_t)c);
+  } else {
+#pragma unroll 1
+    for (uint32_t k = 0; k < len; k++) put(p[k]);
+  }
+  if (n & 3u) x.word(w);
+  return x.done(n, kind, input);
+}
+
 // Returns the key id, or 0xFFFFFFFF when the table is full (the overflow flag
 // is raised and the run is repeated with a bigger table).
-__device__ uint32_t group_find_or_insert(const ScanParams &sp, const KeyRef &k, uint32_t h) {
+__device__ __noinline__ uint32_t group_find_or_insert(const ScanParams &sp, const KeyRef &k, uint32_t h) {
   const GroupTable &g = sp.g;
   uint32_t pos = h & g.cap_mask;
   uint32_t mine = 0xFFFFFFFFu;
@@ -544,6 +683,36 @@ __device__ __forceinline__ unsigned long long group_extreme(unsigned grp, bool o
   return ((unsigned long long)eh << 32) | el;
 }
 
+// Adds the warp's fractional values (of the lanes with `on`) to the limbs in
+// the CTA's shared memory.  Values of like magnitude start at the same limb:
+// then each of their three parts is summed in the warp (a part's 64 bits as
+// two 16-bit pieces and a sign, which cannot overflow over 32 lanes) and one
+// lane adds the sums; adding lane by lane, every lane waits for the others at
+// the same three limbs (avg over 500 MB of lines: 499 us so, 390 reduced).
+__device__ __forceinline__ void warp_fix_add(long long *limbs, double *big, bool on, double v, int lane) {
+  FixParts pr;
+  pr.d = -1;
+  if (on) pr = fix_split(v);
+  const unsigned m = __ballot_sync(0xffffffffu, pr.d != -1);
+  if (!m) return;
+  const int d = __shfl_sync(0xffffffffu, pr.d, __ffs(m) - 1);
+  if (d >= 0 && d + 2 < kFixDigits && __all_sync(0xffffffffu, pr.d == -1 || pr.d == d)) {
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      const unsigned long long u = pr.d == -1 ? 0ull : (unsigned long long)pr.part[k];
+      const uint32_t lo = __reduce_add_sync(0xffffffffu, (uint32_t)u & 0xFFFFu);
+      const uint32_t hi = __reduce_add_sync(0xffffffffu, (uint32_t)u >> 16);
+      const uint32_t neg = __popc(__ballot_sync(0xffffffffu, (long long)u < 0));
+      if (lane == 0)
+        limbs[d + k] += (long long)((unsigned long long)lo + ((unsigned long long)hi << 16) -
+                                    ((unsigned long long)neg << 32));
+    }
+  } else if (on) {
+    fix_atomic_add(limbs, big, v);
+  }
+  __syncwarp();
+}
+
 // One-CTA mbarrier (a tile's bulk copy completes on it) and the 1-D bulk
 // (TMA) copy from this GPU's own global memory into shared memory.  The
 // copy is single-CTA, with no cluster multicast.
@@ -669,7 +838,9 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   Template *tmpl = (Template *)(acc + 1);                           // the run's line template, once seen
   unsigned long long *s_bar = (unsigned long long *)(tmpl + 1);      // tile copies' mbarrier
   uint16_t *lstart = (uint16_t *)(s_bar + 1);                       // kMaxLinesPerPass + 2
-  GroupCache *gcache = (GroupCache *)(smem + scan_smem_base(T, H));  // grouped aggregates only
+  KeyCache *kcache = (KeyCache *)(smem + scan_smem_base(T, H));      // grouped aggregates only
+  const bool whole = P.agg_kind == WARPJQ_AGG_SUM || P.agg_kind == WARPJQ_AGG_AVG;
+  const uint32_t n_places = whole ? kKeyCache / 2 : kKeyCache;
 
   const int lane = threadIdx.x;
   const uint32_t rec_stride = sp.rec_stride;
@@ -686,13 +857,9 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   if (lane < kFixDigits) cta_fix[lane] = 0;
   if (lane == 0) acc->clear();
   const bool grouped = kGroups && !kRows && P.group_slot >= 0;
-  if (grouped) {
-#pragma unroll 1
-    for (int k = lane; k < kGroupCache; k += 32) {
-      gcache->tag[k] = 0xFFFFFFFFu;
-      group_acc_init(gcache->acc[k]);
-    }
-  }
+  if (grouped) keys_clear(*kcache, whole, lane);
+  uint32_t fold_lines = 0;  // lines added to kcache's 32-bit sums since the last fold
+  uint32_t key_input = 0;  // the batch input whose keys kcache holds
   const uint32_t bar = (uint32_t)__cvta_generic_to_shared(s_bar);
   if (lane == 0) mbar_init(bar);
   __syncwarp();
@@ -724,6 +891,12 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       data_end = sp.in_end[input];
       ts = data_start + (tile - sp.in_tile0[input]) * T;
       ctr_in = sp.in_ctr + input;
+      if (kGroups && input != key_input) {
+        keys_flush(*kcache, sp.g, whole, lane);
+        keys_clear(*kcache, whole, lane);
+        key_input = input;
+        fold_lines = 0;
+      }
     }
     const uint32_t nf = P.output_kind == 2 ? P.n_fields : (P.output_kind == 1 ? 1u : 0u);
     const unsigned long long te = min(ts + T, data_end);
@@ -889,7 +1062,9 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
         uint32_t line_len = 0;
         bool has_group = false;
         KeyRef gk;
-        uint32_t gh = 0;
+        uint32_t gh = 0, key_off = 0;  // the key's hash; its window offset
+        uint32_t kw[kKeyCacheBytes / 4];  // a short key's bytes
+        bool odd_key = false;  // escaped, long, or of a line outside the window
         SlotVal aggv;
         aggv.kind = JK_MISSING;
         if (li < cnt) {
@@ -1023,9 +1198,18 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
                 gk.len = g.len;
                 gk.abs_off = line_abs + g.off;
               }
-              gh = (gk.kind == JK_STR ? hash_str_body(gk.p, gk.len, gk.esc) : hash_raw(gk.p, gk.len)) ^
-                   (gk.kind * 0x9E3779B9u) ^ (input * 0x85EBCA6Bu);
-              if (gh == 0) gh = 1;
+              odd_key = !found || gk.esc || gk.len > kKeyCacheBytes;
+              key_off = (uint32_t)(gk.abs_off - ts);
+              if (odd_key) {
+                gh = hash_key_far(gk.p, gk.len, gk.esc, gk.kind, input);
+              } else {
+                KeyHasher x;
+                key_words(win, key_off, gk.len, kw);
+#pragma unroll
+                for (uint32_t k = 0; k < kKeyCacheBytes / 4; k++)
+                  if (4 * k < gk.len) x.word(kw[k]);
+                gh = x.done(gk.len, gk.kind, input);
+              }
             }
           }
         }
@@ -1074,8 +1258,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
             group_sum128(full, ung && is_num && is_int, iv, s_lo, s_hi);
           if (m_num && (ak == WARPJQ_AGG_MIN || ak == WARPJQ_AGG_MAX))
             ext = group_extreme(full, ung && is_num, order_bits(fv), ak == WARPJQ_AGG_MIN);
-          if (ung && is_num && !is_int && (ak == WARPJQ_AGG_SUM || ak == WARPJQ_AGG_AVG))
-            fix_atomic_add(cta_fix, &ctr_in->fbig, fv);  // exact, in the CTA's shared limbs
+          if (ak == WARPJQ_AGG_SUM || ak == WARPJQ_AGG_AVG)
+            warp_fix_add(cta_fix, &ctr_in->fbig, ung && is_num && !is_int, fv, lane);  // exact, in the CTA's limbs
           if (lane == 0) {
             if (m_saw) acc->saw = 1;
             if (m_num) {
@@ -1092,66 +1276,137 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
           }
         }
         if (kGroups && !kRows && P.group_slot >= 0) {
-          // Lanes whose keys hash alike compare their key bytes with the
-          // lowest such lane; only lanes that differ from it look up the
-          // table themselves.
-          const uint32_t hv = has_group ? gh : 0u;
-          const unsigned peers = __match_any_sync(0xffffffffu, hv);
-          const int leader = __ffs(peers) - 1;
-          const unsigned long long lp = __shfl_sync(0xffffffffu, (unsigned long long)gk.p, leader);
-          const uint32_t llen = __shfl_sync(0xffffffffu, gk.len, leader);
-          const uint32_t lkind = __shfl_sync(0xffffffffu, (uint32_t)gk.kind, leader);
-          const uint32_t lesc = __shfl_sync(0xffffffffu, (uint32_t)gk.esc, leader);
-          const uint32_t linput = __shfl_sync(0xffffffffu, input, leader);
-          const bool same = has_group && lane != leader && gk.kind == lkind && input == linput &&
-                            key_bytes_equal(gk, (const uint8_t *)lp, llen, (uint8_t)lesc);
-          uint32_t kid = 0xFFFFFFFFu;
-          if (has_group && !same) kid = group_find_or_insert(sp, gk, gh);
-          const uint32_t lkid = __shfl_sync(0xffffffffu, kid, leader);
-          if (same) kid = lkid;
-          // Lanes holding the same key add up their contributions in the
-          // warp first; one lane per key then updates its accumulators
-          // (counts, the exact integer sum, min or max).  Fractional values
-          // go in per lane, exactly (fixsum.cuh).
-          const unsigned grp = __match_any_sync(0xffffffffu, kid);
-          const bool lead = kid != 0xFFFFFFFFu && lane == __ffs(grp) - 1;
-          const bool num_int = is_num && is_int;
-          const unsigned m_num = __ballot_sync(0xffffffffu, is_num) & grp;
-          const unsigned m_int = __ballot_sync(0xffffffffu, num_int) & grp;
-          const uint32_t ak = P.agg_kind;
-          unsigned long long s_lo = 0, s_hi = 0, ext = 0;
-          if ((ak == WARPJQ_AGG_SUM || ak == WARPJQ_AGG_AVG) && __any_sync(0xffffffffu, num_int))
-            group_sum128(grp, num_int, iv, s_lo, s_hi);
-          if ((ak == WARPJQ_AGG_MIN || ak == WARPJQ_AGG_MAX) && __any_sync(0xffffffffu, is_num))
-            ext = group_extreme(grp, is_num, order_bits(fv), ak == WARPJQ_AGG_MIN);
-          if (kid != 0xFFFFFFFFu && (lead || (is_num && !is_int))) {  // no key id: the table is full
-            // This CTA's cached entry for the key if it has (or can claim)
-            // one, else the global record.
-            GroupAcc *ap = &sp.g.acc[kid];
-            const uint32_t e = kid & (kGroupCache - 1);
-            uint32_t t = *(volatile uint32_t *)&gcache->tag[e];
-            if (t == 0xFFFFFFFFu) {
-              const uint32_t prev = atomicCAS(&gcache->tag[e], 0xFFFFFFFFu, kid);
-              t = prev == 0xFFFFFFFFu ? kid : prev;
+          // A short key is looked up among the CTA's own first.
+          constexpr uint32_t kNone = 0xFFFFFFFFu;
+          uint32_t kid = kNone, ke = kNone;  // the key's id; its place in kcache
+          const uint32_t meta = gk.len | (uint32_t)gk.kind << 24;
+          if (has_group && !odd_key) {
+#pragma unroll 1
+            for (uint32_t j = 0; j < n_places; j++) {
+              const uint32_t e = (gh + j) & (n_places - 1u), hv = kcache->hash[e];
+              if (!hv) break;
+              if (hv != gh || kcache->meta[e] != meta) continue;
+              uint32_t diff = 0;
+#pragma unroll
+              for (uint32_t k = 0; k < kKeyCacheBytes / 4; k++) diff |= kcache->bytes[e][k] ^ kw[k];
+              if (!diff) {
+                kid = kcache->kid[e];
+                ke = e;
+                break;
+              }
             }
-            if (t == kid) ap = &gcache->acc[e];
-            GroupAcc &a = *ap;
-            if (lead) {
-              atomicAdd(&a.count, (unsigned long long)__popc(grp));
-              if (m_num) atomicAdd(&a.numeric, (unsigned long long)__popc(m_num));
-              if (m_int) {
-                atomicAdd(&a.n_int, (unsigned long long)__popc(m_int));
-                if (s_lo || s_hi) {
-                  const unsigned long long old = atomicAdd(&a.isum_lo, s_lo);
-                  const unsigned long long carry = (old + s_lo) < old ? 1ull : 0ull;
-                  if (s_hi + carry) atomicAdd(&a.isum_hi, s_hi + carry);
+          }
+          const bool look = has_group && kid == kNone;
+          if (__any_sync(0xffffffffu, look)) {
+            // Lanes whose keys hash alike compare their key bytes with the
+            // lowest such lane; only lanes that differ from it look up the
+            // table themselves.
+            const unsigned peers = __match_any_sync(0xffffffffu, look ? gh : 0u);
+            const int leader = __ffs(peers) - 1;
+            const unsigned long long lp = __shfl_sync(0xffffffffu, (unsigned long long)gk.p, leader);
+            const uint32_t lmeta = __shfl_sync(0xffffffffu, meta, leader);
+            const uint32_t llen = __shfl_sync(0xffffffffu, gk.len, leader);
+            const uint32_t lesc = __shfl_sync(0xffffffffu, (uint32_t)gk.esc, leader);
+            const bool same = look && lane != leader && gk.kind == lmeta >> 24 &&
+                              key_bytes_equal(gk, (const uint8_t *)lp, llen, (uint8_t)lesc);
+            if (look && !same) {
+              kid = group_find_or_insert(sp, gk, gh);
+              if (!odd_key && kid != kNone) {  // kept in the first free of its places
+#pragma unroll 1
+                for (uint32_t j = 0; j < n_places; j++) {
+                  const uint32_t e = (gh + j) & (n_places - 1u);
+                  if (atomicCAS(&kcache->hash[e], 0u, gh) != 0u) continue;
+#pragma unroll
+                  for (uint32_t k = 0; k < kKeyCacheBytes / 4; k++) kcache->bytes[e][k] = kw[k];
+                  kcache->meta[e] = meta;
+                  kcache->kid[e] = kid;
+                  ke = e;
+                  break;
                 }
               }
-              if (m_num && ak == WARPJQ_AGG_MIN) atomicMin(&a.min_bits, ext);
-              if (m_num && ak == WARPJQ_AGG_MAX) atomicMax(&a.max_bits, ext);
             }
-            if (is_num && !is_int && (ak == WARPJQ_AGG_SUM || ak == WARPJQ_AGG_AVG))
-              fix_atomic_add(a.fix, &a.fbig, fv);
+            const uint32_t lkid = __shfl_sync(0xffffffffu, kid, leader), lke = __shfl_sync(0xffffffffu, ke, leader);
+            if (same) {
+              kid = lkid;
+              ke = lke;
+            }
+          }
+          const uint32_t ak = P.agg_kind;
+          const bool minmax = ak == WARPJQ_AGG_MIN || ak == WARPJQ_AGG_MAX;
+          const bool plain = !has_group || (ke != kNone && (!is_num || minmax || (is_int && iv >= 0 && iv < (1ll << 31))));
+          if (__all_sync(0xffffffffu, plain)) {
+            if (has_group) {
+              atomicAdd(&kcache->n[ke], 1u);
+              if (is_num) {
+                atomicAdd(&kcache->num[ke], 1u);
+                if (minmax) {
+                  if (is_int) atomicAdd(&kcache->lo[ke], 1u);
+                  // few values still move a key's extreme
+                  GroupAcc &a = kcache->at(ke, false);
+                  const unsigned long long ob = order_bits(fv);
+                  if (ak == WARPJQ_AGG_MIN) {
+                    if (ob < a.min_bits) atomicMin(&a.min_bits, ob);
+                  } else if (ob > a.max_bits) {
+                    atomicMax(&a.max_bits, ob);
+                  }
+                } else {
+                  atomicAdd(&kcache->lo[ke], (uint32_t)iv & 0xFFFFu);
+                  atomicAdd(&kcache->hi[ke], (uint32_t)iv >> 16);
+                }
+              }
+            }
+            if ((fold_lines += 32) >= kFoldLines) {
+              keys_fold(*kcache, whole, lane);
+              fold_lines = 0;
+            }
+          } else {
+            // Lanes holding the same key add up their contributions in the
+            // warp first; one lane per key then updates its accumulators
+            // (counts, the exact integer sum, min or max).  Fractional values
+            // go in per lane, exactly (fixsum.cuh).  kcache's are this warp's,
+            // and one lane of it leads a key, so its adds need no atomics.
+            const unsigned grp = __match_any_sync(0xffffffffu, kid);
+            const bool lead = kid != kNone && lane == __ffs(grp) - 1;
+            const bool num_int = is_num && is_int;
+            const unsigned m_num = __ballot_sync(0xffffffffu, is_num) & grp;
+            const unsigned m_int = __ballot_sync(0xffffffffu, num_int) & grp;
+            unsigned long long s_lo = 0, s_hi = 0, ext = 0;
+            if (whole && __any_sync(0xffffffffu, num_int)) group_sum128(grp, num_int, iv, s_lo, s_hi);
+            if (minmax && __any_sync(0xffffffffu, is_num))
+              ext = group_extreme(grp, is_num, order_bits(fv), ak == WARPJQ_AGG_MIN);
+            const bool frac = is_num && !is_int && whole;
+            if (kid == kNone) {  // no key, or the table is full
+            } else if (ke != kNone) {
+              GroupAcc &a = kcache->at(ke, whole);
+              if (lead) {
+                a.count += __popc(grp);
+                a.numeric += __popc(m_num);
+                a.n_int += __popc(m_int);
+                const unsigned long long lo = a.isum_lo + s_lo;
+                a.isum_hi += s_hi + (lo < s_lo ? 1ull : 0ull);
+                a.isum_lo = lo;
+                if (m_num && ak == WARPJQ_AGG_MIN) a.min_bits = min(a.min_bits, ext);
+                if (m_num && ak == WARPJQ_AGG_MAX) a.max_bits = max(a.max_bits, ext);
+              }
+              if (frac) fix_atomic_add(a.fix, &a.fbig, fv);
+            } else {
+              GroupAcc &a = sp.g.acc[kid];
+              if (lead) {
+                atomicAdd(&a.count, (unsigned long long)__popc(grp));
+                if (m_num) atomicAdd(&a.numeric, (unsigned long long)__popc(m_num));
+                if (m_int) {
+                  atomicAdd(&a.n_int, (unsigned long long)__popc(m_int));
+                  if (s_lo || s_hi) {
+                    const unsigned long long old = atomicAdd(&a.isum_lo, s_lo);
+                    const unsigned long long carry = (old + s_lo) < old ? 1ull : 0ull;
+                    if (s_hi + carry) atomicAdd(&a.isum_hi, s_hi + carry);
+                  }
+                }
+                if (m_num && ak == WARPJQ_AGG_MIN) atomicMin(&a.min_bits, ext);
+                if (m_num && ak == WARPJQ_AGG_MAX) atomicMax(&a.max_bits, ext);
+              }
+              if (frac) fix_atomic_add(a.fix, &a.fbig, fv);
+            }
           }
           if (kid != 0xFFFFFFFFu && !is_num && aggv.kind != JK_MISSING && aggv.kind != JK_NULL &&
               P.agg_slot >= 0)
@@ -1225,35 +1480,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       flush_counts(ctr_in, sp.ctr, P, kRows, lane, acc, cta_fix);
   }
 
-  // Merge this CTA's cached group accumulators into the global records.
-  if (grouped) {
-    __syncwarp();
-#pragma unroll 1
-    for (int k = lane; k < kGroupCache; k += 32) {
-      const uint32_t kid = gcache->tag[k];
-      if (kid == 0xFFFFFFFFu) continue;
-      const GroupAcc c = gcache->acc[k];
-      GroupAcc &a = sp.g.acc[kid];
-      if (c.count) atomicAdd(&a.count, c.count);
-      if (c.numeric) {
-        atomicAdd(&a.numeric, c.numeric);
-        atomicMin(&a.min_bits, c.min_bits);
-        atomicMax(&a.max_bits, c.max_bits);
-      }
-      if (c.n_int) {
-        const unsigned long long old = atomicAdd(&a.isum_lo, c.isum_lo);
-        const unsigned long long carry = (old + c.isum_lo) < old ? 1ull : 0ull;
-        if (c.isum_hi + carry) atomicAdd(&a.isum_hi, c.isum_hi + carry);
-        atomicAdd(&a.n_int, c.n_int);
-      }
-      if (c.numeric > c.n_int) {
-#pragma unroll 1
-        for (int d = 0; d < kFixDigits; d++)
-          if (c.fix[d]) atomicAdd((unsigned long long *)&a.fix[d], (unsigned long long)c.fix[d]);
-        if (c.fbig != 0.0) atomicAdd(&a.fbig, c.fbig);
-      }
-    }
-  }
+  // Merge this CTA's own group accumulators into the global records.
+  if (grouped) keys_flush(*kcache, sp.g, whole, lane);
 
   if (kRows && sp.rec_cursor && lane == 0) sp.rec_cursor[blockIdx.x] = cta_recs;
   // Flush this CTA's counters (a batch's were flushed per tile).
