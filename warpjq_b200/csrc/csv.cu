@@ -29,9 +29,9 @@
 //   k_csv_tiles     one block: each tile's start state and first row
 //   k_csv_row_ends  each row's end offset
 //   k_csv_close     the last row, the consumed length, the header's end
-//   k_csv_json<0>   one thread per row: its NDJSON length
+//   k_csv_json<0>   every row's NDJSON length, 32 rows a warp
 //   (exclusive scan of the lengths)
-//   k_csv_json<1>   one thread per row: its NDJSON bytes
+//   k_csv_json<1>   every row's NDJSON bytes, 32 rows a warp
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -46,6 +46,11 @@
 #include "../../include/warpjq_ext.h"
 #include "csv_rows.cuh"
 
+// The window helpers of the scan, with internal linkage.
+namespace {
+#include "walker.cuh"
+}
+
 using namespace wjq_csv;
 
 namespace {
@@ -54,7 +59,6 @@ constexpr uint32_t kRun = 256;                     // bytes a thread owns in the
 constexpr int kCsvThreads = 256;                   // threads per tile
 constexpr uint32_t kCsvTile = kRun * kCsvThreads;  // 64 KiB
 constexpr int kScanBlock = 1024;                   // elements per block of the u64 scan
-constexpr int kJsonThreads = 128;
 
 void csv_err(char *err, size_t len, const char *fmt, ...) {
   if (!err || !len) return;
@@ -223,22 +227,279 @@ __global__ void k_csv_close(u64 *row_end, u64 n, int final_, u64 *info) {
   info[2] = r ? row_end[0] : 0;
 }
 
-// Rows [row0, rows) of the chunk, one thread each: pass 0 writes the NDJSON
-// length of line r - row0 to len_off, pass 1 writes the line at out +
-// len_off[r - row0] (len_off by then an exclusive prefix).
-template <bool kWrite>
-__global__ void __launch_bounds__(kJsonThreads) k_csv_json(const uint8_t *d, const u64 *row_end, u64 row0,
-                                                           u64 rows, KeySet ks, u64 *len_off, uint8_t *out) {
-  for (u64 r = row0 + blockIdx.x * (u64)blockDim.x + threadIdx.x; r < rows; r += (u64)gridDim.x * blockDim.x) {
-    const u64 s = r ? __ldg(row_end + r - 1) + 1 : 0, e = __ldg(row_end + r);
-    WordIn in(d);
-    if (!kWrite) {
-      WordOut w(nullptr);
-      len_off[r - row0] = row_json<false>(in, s, e, ks, w);
+// Rows to NDJSON, 32 rows a warp (one warp a block), a lane a row.  The rows'
+// bytes are staged in shared memory (they are contiguous, so the loads are
+// whole blocks), and every 32 of them become a mask of the bytes a row's walk
+// has to look at: ',' '"' '\\' and control bytes.  A lane then steps from hit
+// to hit, takes a field's kind from its first byte and its end, and moves
+// everything else a word at a time; the lines, contiguous too, are put
+// together in shared memory and written out as whole blocks.  A thread a row
+// over global memory, stepping a word at a time through every byte, was bound
+// by its instructions: 256 MB of CSV took 762 us for the lengths and 1,111 us
+// for the bytes; 179 and 783 so.  What bounds the second now is latency: 14 KB
+// of windows leave 15 warps an SM, and the lanes' escapes fall on different
+// bytes.  (Copying short pieces byte by byte took 857, byte by byte through
+// the fields with escapes 938.)
+constexpr uint32_t kCsvWin = 5120;   // staged input bytes
+constexpr uint32_t kCsvOut = 8192;   // staged output bytes
+constexpr uint32_t kCsvMask = kCsvWin / 32 + 2;
+constexpr uint32_t kCsvOff = kCsvWin + 64 + (kCsvMask * 4 + 15) / 16 * 16;  // where the output starts
+
+__host__ __device__ constexpr uint32_t csv_smem(bool write) { return kCsvOff + (write ? kCsvOut + 16 : 0u); }
+
+// The hits of eight words: ',' '"' '\\' and bytes below 0x20 (devutil.cuh
+// flags_special, with ',').
+__device__ __forceinline__ uint32_t csv_hits(const uint32_t w[8]) {
+  uint32_t m = 0;
+#pragma unroll
+  for (int k = 7; k >= 0; k--) {
+    const uint32_t t = (w[k] ^ 0x02020202u) & 0x7F7F7F7Fu;
+    const uint32_t sq = t + 0x5F5F5F5Fu, sb = (t ^ 0x5E5E5E5Eu) + 0x7F7F7F7Fu, sc = (t ^ 0x2E2E2E2Eu) + 0x7F7F7F7Fu;
+    m = wjq::flags_push(m, ~((sq & sb & sc) | w[k]) & 0x80808080u);
+  }
+  return m;
+}
+
+// Output into shared memory from byte `at` on, a word at a time; the words a
+// line shares with its neighbours are written bytewise.
+struct LineOut {
+  uint32_t *o;
+  uint32_t first;   // the word the line starts in, when it starts within it
+  uint32_t skip;    // that word's bytes before the line
+  uint32_t w, off;  // the word being filled, its bytes so far
+  uint32_t acc;     // and those
+  __device__ __forceinline__ LineOut(uint32_t *o_, uint32_t at)
+      : o(o_), first(at & 3 ? at >> 2 : 0xFFFFFFFFu), skip(at & 3), w(at >> 2), off(at & 3), acc(0) {}
+  __device__ __forceinline__ void bytes(uint32_t x, uint32_t n) {  // bytes up to n of word w
+    for (uint32_t j = w == first ? skip : 0u; j < n; j++) ((uint8_t *)o)[4 * w + j] = (uint8_t)(x >> (8 * j));
+  }
+  __device__ __forceinline__ void put(uint32_t v, uint32_t k) {  // the k (1..4) low bytes of v, the others zero
+    const uint32_t x = acc | v << (8 * off);
+    const uint32_t n = off + k;
+    if (n < 4) {
+      acc = x;
+      off = n;
     } else {
-      WordOut w(out + len_off[r - row0]);
-      row_json<true>(in, s, e, ks, w);
-      w.flush();
+      if (w == first) bytes(x, 4);
+      else o[w] = x;
+      w++;
+      acc = __funnelshift_l(v, 0u, 8 * off);  // what did not fit
+      off = n - 4;
+    }
+  }
+  __device__ __forceinline__ void flush() { bytes(acc, off); }
+  // Bytes [a, b) of the window: up to the next word of the output, then whole
+  // words straight across, then the rest.
+  __device__ __forceinline__ void copy(const uint8_t *win, uint32_t a, uint32_t b) {
+    if (off && a < b) {
+      const uint32_t k = min(4 - off, b - a);
+      put(wjq::detail::load4(win, a) & (0xFFFFFFFFu >> (32 - 8 * k)), k);
+      a += k;
+    }
+    if (a >= b) return;
+    const uint32_t *q = (const uint32_t *)win + (a >> 2);
+    const uint32_t sh = (a & 3u) * 8u;
+    uint32_t lo = *q;
+#pragma unroll 1
+    for (; a + 4 <= b; a += 4) {
+      const uint32_t hi = *++q;
+      o[w++] = __funnelshift_r(lo, hi, sh);
+      lo = hi;
+    }
+    off = b - a;
+    acc = off ? __funnelshift_r(lo, q[1], sh) & (0xFFFFFFFFu >> (32 - 8 * off)) : 0u;
+  }
+  __device__ __forceinline__ void escape(uint32_t c) {
+    const uint32_t two = c == '\n' ? 'n' : c == '\r' ? 'r' : c == '\t' ? 't' : c == 8 ? 'b' : c == 12 ? 'f'
+                         : c >= 0x20 ? c : 0u;
+    if (two) {
+      put('\\' | two << 8, 2);
+    } else {
+      const uint32_t l = c & 15;
+      put('\\' | 'u' << 8 | '0' << 16 | (uint32_t)'0' << 24, 4);
+      put((uint32_t)('0' + (c >> 4)) | (uint32_t)(l < 10 ? '0' + l : 'a' + l - 10) << 8, 2);
+    }
+  }
+};
+
+// One row w[s, e) of a window (hits in sm; w[e] is a hit): its NDJSON length,
+// and with kWrite its bytes.  0 for a row with bytes after a field's closing
+// quote, which row_json takes.  The fields' rules are row_json's.
+template <bool kWrite>
+__device__ __forceinline__ uint32_t row_line(const uint8_t *w, const uint32_t *sm, uint32_t s, uint32_t e, bool on,
+                                             const KeySet &ks, LineOut &o) {
+  if (on && e > s && w[e - 1] == '\r') e--;
+  const bool empty = e == s;
+  uint32_t len = 3, p = s;  // "{" "}\n"
+  bool more = on && !empty, odd = false;
+  if (kWrite && more) o.put('{', 1);
+#pragma unroll 1
+  for (uint32_t k = 0; k < ks.n && __any_sync(0xffffffffu, more); k++) {
+    const uint32_t kw = __ldg(ks.meta + 2 * k), kl = __ldg(ks.meta + 2 * k + 1);
+    if (more) {
+      len += kl;
+      if (kWrite)
+#pragma unroll 1
+        for (uint32_t j = 0; j < kl; j += 4) o.put(__ldg(ks.text + kw + (j >> 2)), min(kl - j, 4u));
+    }
+    __syncwarp();
+    // the field's text [a, b), and whether it holds bytes to escape
+    const uint32_t c = more && p < e ? w[p] : 0u;
+    const bool quoted = c == '"';
+    const uint32_t a = quoted ? p + 1 : p;
+    uint32_t b = a, extra = 0;
+    bool esc = false, go = more;
+#pragma unroll 1
+    while (go) {
+      b = min(wjq::detail::next_special(sm, b), e);
+      const uint32_t x = w[b];
+      if (b == e) {
+        go = false;
+      } else if (x == ',') {
+        go = quoted;
+        b += quoted;
+      } else if (x != '"') {
+        esc = true;
+        extra += esc_len((uint8_t)x) - 1;
+        b++;
+      } else if (!quoted) {
+        esc = true;
+        extra++;
+        b++;
+      } else if (b + 1 < e && w[b + 1] == '"') {  // a doubled quote stays two bytes
+        esc = true;
+        b += 2;
+      } else {
+        go = false;
+      }
+    }
+    __syncwarp();
+    if (more) {
+      p = quoted && b < e ? b + 1 : b;  // past the closing quote
+      if (quoted && p < e && w[p] != ',') odd = true;
+      const bool null = !quoted && b == a;
+      const bool number = !quoted && !esc && !null && (c == '-' || c - '0' < 10u) && wjq::detail::win_number(w, a, c) == b;
+      const bool str = !null && !number;
+      len += null ? 4u : b - a + extra + (str ? 2u : 0u);
+      if (kWrite) {
+        if (null) o.put('n' | 'u' << 8 | 'l' << 16 | (uint32_t)'l' << 24, 4);
+        if (str) o.put('"', 1);
+        uint32_t q = a;
+#pragma unroll 1
+        while (esc && q < b) {
+          const uint32_t h = min(wjq::detail::next_special(sm, q), b);
+          o.copy(w, q, h);
+          q = h;
+          if (h < b) {
+            const uint32_t x = w[h];
+            if (x == ',') o.put(',', 1);
+            else o.escape(x);
+            q += x == '"' && quoted ? 2 : 1;
+          }
+        }
+        if (!esc && !null) o.copy(w, a, b);
+        if (str) o.put('"', 1);
+      }
+      more = p < e && !odd;  // a ',' follows
+      p++;
+    }
+    __syncwarp();
+  }
+  if (kWrite && on) {
+    if (empty) o.put('\n', 1);
+    else o.put('}' | '\n' << 8, 2);
+    o.flush();
+  }
+  return odd ? 0u : empty ? 1u : len;
+}
+
+// Rows [row0, rows) of the chunk: pass 0 writes the NDJSON length of line r -
+// row0 to len_off, pass 1 writes the line at out + len_off[r - row0] (len_off
+// by then an exclusive prefix, *total the end of the last line).  A warp takes
+// as many of its 32 rows at once as fit the staged windows; a row that fits
+// none alone, or has bytes after a closing quote, goes by row_json.
+template <bool kWrite>
+__global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *row_end, u64 row0, u64 rows, KeySet ks,
+                                                 u64 *len_off, uint8_t *out, const u64 *total) {
+  extern __shared__ __align__(16) uint8_t csv_sm[];
+  uint8_t *win = csv_sm;
+  uint32_t *mask = (uint32_t *)(csv_sm + kCsvWin + 64);
+  uint32_t *obuf = (uint32_t *)(csv_sm + kCsvOff);
+  const uint32_t lane = threadIdx.x;
+  for (u64 base = row0 + blockIdx.x * 32ull; base < rows; base += gridDim.x * 32ull) {
+    const u64 r = base + lane;
+    const uint32_t n_here = (uint32_t)min((u64)32, rows - base);
+    const bool mine = lane < n_here;
+    u64 s = 0, e = 0, o0 = 0, o1 = 0;  // the row, and its line in the output
+    if (mine) {
+      s = r ? __ldg(row_end + r - 1) + 1 : 0;
+      e = __ldg(row_end + r);
+      if (kWrite) {
+        o0 = len_off[r - row0];
+        o1 = r + 1 < rows ? len_off[r + 1 - row0] : *total;
+      }
+    }
+    for (uint32_t lo = 0; lo < n_here;) {
+      const u64 s_lo = __shfl_sync(0xffffffffu, s, lo), o_lo = __shfl_sync(0xffffffffu, o0, lo);
+      const u64 w0 = (u64)((uintptr_t)(d + s_lo) & 15u);  // the window starts at a block
+      const uint32_t lead = (uint32_t)((uintptr_t)(out + o_lo) & 15u);
+      const bool fits = mine && lane >= lo && e - s_lo + w0 < kCsvWin && (!kWrite || o1 - o_lo + lead <= kCsvOut);
+      const unsigned m = __ballot_sync(0xffffffffu, fits) >> lo;
+      const uint32_t take = m == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~m) - 1u;  // rows lo .. lo + take fit
+      const bool on = fits && lane < lo + take;
+      if (take) {
+        const uint32_t hi = lo + take - 1;
+        const uint32_t n_win = (uint32_t)(__shfl_sync(0xffffffffu, e, hi) - s_lo + w0);
+        const uint4 *src = (const uint4 *)((uintptr_t)(d + s_lo) & ~(uintptr_t)15);
+        // whole blocks, each holding a byte of the rows
+        for (uint32_t k = lane; 16 * k < n_win; k += 32) ((uint4 *)win)[k] = __ldg(src + k);
+        __syncwarp();
+        if (lane == 0) win[n_win] = '\n';  // ends the last row
+        __syncwarp();
+        for (uint32_t k = lane; 32 * k <= n_win; k += 32) {
+          const uint4 u = ((const uint4 *)win)[2 * k], v = ((const uint4 *)win)[2 * k + 1];
+          const uint32_t w8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+          mask[k] = csv_hits(w8);
+        }
+        __syncwarp();
+        const uint32_t ws = on ? (uint32_t)(s - s_lo + w0) : 0u, we = on ? (uint32_t)(e - s_lo + w0) : 0u;
+        const uint32_t at = on ? (uint32_t)(o0 - o_lo) + lead : 0u;
+        LineOut o(obuf, at);
+        uint32_t len = row_line<kWrite>(win, mask, ws, we, on, ks, o);
+        if (on && !len) {  // row_json takes it
+          WordIn in(d);
+          WordOut wo(kWrite ? (uint8_t *)obuf + at : nullptr);
+          len = (uint32_t)row_json<kWrite>(in, s, e, ks, wo);
+          if (kWrite) wo.flush();
+        }
+        __syncwarp();
+        if (!kWrite) {
+          if (on) len_off[r - row0] = len;
+        } else {
+          // whole blocks, and the bytes around them
+          const uint32_t end = (uint32_t)(__shfl_sync(0xffffffffu, o1, hi) - o_lo) + lead;
+          uint8_t *dst = out + o_lo - lead;
+          for (uint32_t k = 16 * lane; k < end; k += 512) {
+            if (k >= lead && k + 16 <= end) {
+              *(uint4 *)(dst + k) = *(const uint4 *)((const uint8_t *)obuf + k);
+            } else {
+              for (uint32_t j = max(k, lead); j < min(k + 16, end); j++) dst[j] = ((const uint8_t *)obuf)[j];
+            }
+          }
+          __syncwarp();
+        }
+        lo += take;
+      } else {  // row lo is too long for the windows
+        if (lane == lo) {
+          WordIn in(d);
+          WordOut wo(kWrite ? out + o0 : nullptr);
+          const u64 len = row_json<kWrite>(in, s, e, ks, wo);
+          if (kWrite) wo.flush();
+          else len_off[r - row0] = len;
+        }
+        __syncwarp();
+        lo++;
+      }
     }
   }
 }
@@ -450,8 +711,8 @@ warpjq_status warpjq_csv_convert(warpjq_csv *c, const uint8_t *src, uint64_t n, 
   if (m == 0) return WARPJQ_OK;
   KeySet ks{c->keys.p, c->key_off.p, (uint32_t)(c->key_meta.size() / 2)};
   CSV_CK(c->lens.ensure(m + 1), "device memory for CSV lines");
-  const unsigned grid = (unsigned)std::min<u64>((m + kJsonThreads - 1) / kJsonThreads, 148ull * 64);
-  k_csv_json<false><<<grid, kJsonThreads, 0, st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, nullptr);
+  const unsigned grid = (unsigned)std::min<u64>((m + 31) / 32, 148ull * 256);
+  k_csv_json<false><<<grid, 32, csv_smem(false), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, nullptr, nullptr);
   const u64 nb = (m + kScanBlock - 1) / kScanBlock;
   CSV_CK(c->bt.ensure(nb), "device memory for CSV lines");
   k_sum_blocks<<<(unsigned)nb, 256, 0, st>>>(c->lens.p, m, c->bt.p);
@@ -462,7 +723,8 @@ warpjq_status warpjq_csv_convert(warpjq_csv *c, const uint8_t *src, uint64_t n, 
   CSV_CK(cudaMemcpyAsync(&total, c->info.p + 3, 8, cudaMemcpyDeviceToHost, st), "CSV line lengths");
   CSV_CK(cudaStreamSynchronize(st), "CSV line lengths");
   CSV_CK(c->out.ensure(total + 16), "device memory for the NDJSON");
-  k_csv_json<true><<<grid, kJsonThreads, 0, st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, c->out.p);
+  k_csv_json<true><<<grid, 32, csv_smem(true), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, c->out.p,
+                                                     c->info.p + 3);
   CSV_CK(cudaGetLastError(), "CSV to NDJSON");
   *d_ndjson = c->out.p;
   *ndjson_len = total;

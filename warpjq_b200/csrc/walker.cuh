@@ -471,16 +471,10 @@ __device__ __forceinline__ uint32_t mask_string(const uint8_t *w, const uint32_t
   }
 }
 
-// End (exclusive) of the number or literal starting at w[i] == c, or 0 when
-// it is malformed.  The byte after it is checked by the caller.
-__device__ __forceinline__ uint32_t win_atom(const uint8_t *w, uint32_t i, uint32_t c) {
-  if (c > '9') {
-    if (c == 't') return load4(w, i) == 0x65757274u ? i + 4 : 0;      // "true"
-    if (c == 'n') return load4(w, i) == 0x6C6C756Eu ? i + 4 : 0;      // "null"
-    if (c == 'f') return load4(w, i + 1) == 0x65736C61u ? i + 5 : 0;  // "alse"
-    return 0;
-  }
-  // -?(0|[1-9][0-9]*)(\.[0-9]+)?([eE][+-]?[0-9]+)?   (json.rs:370-410)
+// End (exclusive) of the number starting at w[i] == c, or 0 when it is
+// malformed: -?(0|[1-9][0-9]*)(\.[0-9]+)?([eE][+-]?[0-9]+)?  (json.rs:370-410).
+// The byte after it is checked by the caller.
+__device__ __forceinline__ uint32_t win_number(const uint8_t *w, uint32_t i, uint32_t c) {
   uint32_t j = i;
   if (c == '-') c = w[++j];
   if (c - '0' >= 10u) return 0;
@@ -501,6 +495,16 @@ __device__ __forceinline__ uint32_t win_atom(const uint8_t *w, uint32_t i, uint3
     j += d;
   }
   return j;
+}
+
+// End (exclusive) of the number or literal starting at w[i] == c, or 0 when
+// it is malformed.
+__device__ __forceinline__ uint32_t win_atom(const uint8_t *w, uint32_t i, uint32_t c) {
+  if (c <= '9') return win_number(w, i, c);
+  if (c == 't') return load4(w, i) == 0x65757274u ? i + 4 : 0;      // "true"
+  if (c == 'n') return load4(w, i) == 0x6C6C756Eu ? i + 4 : 0;      // "null"
+  if (c == 'f') return load4(w, i + 1) == 0x65736C61u ? i + 5 : 0;  // "alse"
+  return 0;
 }
 
 // match_key for a key body at w[off, off + len) of a window: keys of up to
