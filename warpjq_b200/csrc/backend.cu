@@ -2,8 +2,9 @@
 // (reference crates/warpjq-core/cuda/warpjq_kernels.h:238-274) and the
 // device-resident extension of warpjq_ext.h.
 //
-// Per run the backend launches four kernels on one stream -- reset, scan,
-// tile reduction, finalize -- with no host synchronisation in between.
+// Per run the backend launches three kernels on one stream -- reset, scan and
+// the tail over the tiles, and for rows their copy -- with no host
+// synchronisation in between.
 // Device buffers that depend on the data (row records, output bytes, the
 // group table, the deep-nesting stack) start at a size that fits ordinary
 // input and are grown when the scan reports that one was too small; the run
@@ -95,7 +96,6 @@ struct RunBufs {
   DevBuf<uint8_t> recs;
   DevBuf<uint8_t> out;
   DevBuf<unsigned long long> row_off, line_idx;
-  DevBuf<unsigned long long> block_lines;
   DevBuf<uint32_t> deep;
   DevBuf<TemplateBuf> tmpl;  // a line template per plan of the run
   // group table
@@ -125,12 +125,10 @@ struct RunBufs {
     b_tickets.release();
     b_rec_cursor.release();
     recs.release(); out.release(); row_off.release(); line_idx.release();
-    block_lines.release(); deep.release(); tmpl.release(); g_slots.release();
+    deep.release(); tmpl.release(); g_slots.release();
     g_keys.release(); g_acc.release(); g_ext.release(); g_in.release();
   }
 };
-
-constexpr unsigned kReduceBlocks = 256;
 
 __global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, TemplateBuf *tmpl, uint32_t n_tmpl) {
   unsigned long long tid = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
@@ -287,12 +285,12 @@ warpjq_status ensure_bufs(warpjq_ctx *c, Slot &s, unsigned long long n,
   if (n_tiles == 0) n_tiles = 1;
   CK(rb.ctr.ensure(1, st, cap), "alloc counters");
   CK(rb.tiles.ensure(n_tiles, st, cap), "alloc tiles");
-  CK(rb.block_lines.ensure(2 * kReduceBlocks, st, cap), "alloc reduce");
+  const uint32_t tail_tpb = tail_tiles_per_block(n_tiles, rows);
+  CK(rb.row_bsum.ensure(3ull * tail_blocks(n_tiles, tail_tpb), st, cap), "alloc tile sums");
   if (!rb.deep_levels) rb.deep_levels = 1u << 16;
   CK(rb.deep.ensure((size_t)c->grid * (rb.deep_levels / 32), st, cap), "alloc deep stack");
   if (rows) {
     CK(rb.row_tiles.ensure(n_tiles, st, cap), "alloc row tiles");
-    CK(rb.row_bsum.ensure(3 * ((n_tiles + 7) / 8), st, cap), "alloc row prefixes");
     // Records accumulate over all of a CTA's tiles: room for a row per KiB
     // of input, grown on overflow; output and row capacities follow the
     // input's size too (a larger input than the last does not overflow
@@ -524,13 +522,28 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
       CK(cudaGetLastError(), "launch scan");
     }
     if (s.timed) CK(cudaEventRecord(s.scan_t1, st), "event record");
+    TailParams tp{};
+    tp.n_tiles = n_tiles;
+    tp.tpb = tail_tiles_per_block(n_tiles, rows);
+    tp.tiles = rb.tiles.p;
+    tp.row_tiles = rows ? rb.row_tiles.p : nullptr;
+    tp.bsum = rb.row_bsum.p;
+    tp.ctr = rb.ctr.p;
+    tp.row_off = rb.row_off.p;
+    tp.rows_cap = rb.rows_cap;
+    tp.out_cap = rb.out_cap;
+    if (groups) {
+      tp.keys = rb.g_keys.p;
+      tp.acc = rb.g_acc.p;
+      tp.key_cap = rb.g_key_cap;
+      tp.ext = rb.g_ext.p;
+      tp.ext_input = rb.g_in.p;
+    }
+    const unsigned nb = tail_blocks(n_tiles, tp.tpb);
+    k_tail<<<nb, kTailThreads, 0, st>>>(tp);
+    s.kernels++;
+    CK(cudaGetLastError(), "launch tail");
     if (rows) {
-      const uint32_t tpb = rows_tiles_per_block(n_tiles);
-      const unsigned nb = (unsigned)((n_tiles + tpb - 1) / tpb);
-      k_rows_block_sums<<<nb, kEmitThreads, 0, st>>>(rb.row_tiles.p, rb.tiles.p, n_tiles, tpb,
-                                                      rb.row_bsum.p);
-      k_rows_block_prefix<<<1, kPrefixThreads, 0, st>>>(rb.row_bsum.p, nb, rb.ctr.p, rb.row_off.p,
-                                                      rb.rows_cap, rb.out_cap);
       EmitParams ep{};
       ep.data = d_data;
       ep.rec_stride = sp.rec_stride;
@@ -543,7 +556,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
       ep.tiles = rb.tiles.p;
       ep.n_tiles = n_tiles;
       ep.block_prefix = rb.row_bsum.p;
-      ep.tiles_per_block = tpb;
+      ep.tiles_per_block = tp.tpb;
       ep.recs = rb.recs.p;
       ep.out = rb.out.p;
       ep.out_cap = rb.out_cap;
@@ -553,21 +566,9 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
       ep.ctr = rb.ctr.p;
       if (b && b->mixed) k_rows_emit<true><<<nb, kEmitThreads, 0, st>>>(ep, P);
       else k_rows_emit<false><<<nb, kEmitThreads, 0, st>>>(ep, P);
-      s.kernels += 3;
+      s.kernels++;
       CK(cudaGetLastError(), "launch rows");
     }
-    if (groups) {
-      k_groups_compact<<<(unsigned)std::min<uint32_t>((rb.g_key_cap + 255) / 256, 4u * c->num_sms), 256, 0, st>>>(
-          rb.ctr.p, rb.g_keys.p, rb.g_acc.p, rb.g_key_cap, rb.g_ext.p, rb.g_in.p);
-      s.kernels++;
-    }
-    k_reduce_tiles<<<kReduceBlocks, kReduceThreads, 0, st>>>(n_tiles, rb.tiles.p, rb.ctr.p,
-                                                             rb.block_lines.p);
-    s.kernels++;
-    CK(cudaGetLastError(), "launch reduce");
-    k_finalize<<<1, 32, 0, st>>>(rb.block_lines.p, kReduceBlocks, rb.tiles.p, rb.ctr.p);
-    s.kernels++;
-    CK(cudaGetLastError(), "launch finalize");
     if (b && n_inputs) {
       k_batch_finalize<<<(n_inputs + 7) / 8, 256, 0, st>>>(rb.tiles.p, rb.b_in_tile0.p, rb.b_in_ctr.p,
                                                           n_inputs);
@@ -696,7 +697,6 @@ uint64_t bufs_signature(const warpjq_ctx *c) {
   mix((uintptr_t)rb.recs.p); mix(rb.recs.n);
   mix((uintptr_t)rb.out.p); mix(rb.out.n);
   mix((uintptr_t)rb.row_off.p); mix((uintptr_t)rb.line_idx.p);
-  mix((uintptr_t)rb.block_lines.p);
   mix((uintptr_t)rb.deep.p); mix(rb.deep.n);
   mix((uintptr_t)rb.tmpl.p); mix(rb.tmpl.n);
   mix((uintptr_t)rb.g_slots.p); mix((uintptr_t)rb.g_keys.p); mix((uintptr_t)rb.g_acc.p);

@@ -125,42 +125,35 @@ __host__ __device__ inline double fix_to_double(const long long *limb, unsigned 
       c = s >> 32;
     }
   }
-  int top = -1;  // highest set bit of the magnitude
-  for (int i = 11; i >= 0 && top < 0; i--)
-    if (dg[i]) {
-      int b = 31;
-      while (!((dg[i] >> b) & 1u)) b--;
-      top = 32 * i + b;
-    }
-  if (top < 0) return 0.0;
-  auto bit = [&](int k) -> unsigned { return k < 0 ? 0u : (dg[k >> 5] >> (k & 31)) & 1u; };
-  // 53 significant bits from `top` down, then round to nearest-even with the
-  // rest as guard and sticky bits
-  unsigned long long mant = 0;
-  for (int k = top; k > top - 53; k--) mant = (mant << 1) | bit(k);
-  const int g = top - 53;
+  int i = 11;  // the highest digit with a set bit
+  while (i >= 0 && !dg[i]) i--;
+  if (i < 0) return 0.0;
+  // the top four digits as 128 bits with the highest set bit first, and
+  // whether anything lies below them
+  unsigned __int128 x = 0;
+  for (int k = 0; k < 4; k++) x = x << 32 | (i - k >= 0 ? dg[i - k] : 0u);
   bool sticky = false;
-  for (int k = g - 1; k >= 0 && !sticky; k--) sticky = bit(k) != 0;
-  if (bit(g) && (sticky || (mant & 1))) mant++;
-  int e2 = top - 52 - kFixLowBits;  // value = mant * 2^e2
+  for (int k = i - 4; k >= 0; k--) sticky = sticky || dg[k] != 0;
+  int lead = 0;
+  while (!((dg[i] << lead) >> 31)) lead++;
+  x <<= lead;
+  // 53 significant bits, rounded to nearest-even with the rest as guard and
+  // sticky bits; mant * 2^e2 is in the normal range (|total| < 2^260 and
+  // >= 2^-128), so the result is put together from its fields
+  unsigned long long mant = (unsigned long long)(x >> 75);
+  const unsigned guard = (unsigned)(x >> 74) & 1u;
+  sticky = sticky || (x & ((((unsigned __int128)1) << 74) - 1)) != 0;
+  if (guard && (sticky || (mant & 1))) mant++;
+  int e2 = 32 * i + 31 - lead - 52 - kFixLowBits;  // value = mant * 2^e2
   if (mant >> 53) {
     mant >>= 1;
     e2++;
   }
-  // mant * 2^e2 as a double; every total here is in the normal range
-  // (|total| < 2^260 and >= 2^-128), so the scaling is exact
-  double x = (double)mant;
-  while (e2 > 0) {
-    const int s = e2 > 60 ? 60 : e2;
-    x *= (double)(1ull << s);
-    e2 -= s;
-  }
-  while (e2 < 0) {
-    const int s = -e2 > 60 ? 60 : -e2;
-    x /= (double)(1ull << s);
-    e2 += s;
-  }
-  return neg ? -x : x;
+  const unsigned long long bits =
+      (neg ? 1ull << 63 : 0ull) | (unsigned long long)(e2 + 1075) << 52 | (mant & ((1ull << 52) - 1));
+  double r;
+  __builtin_memcpy(&r, &bits, 8);
+  return r;
 }
 
 }  // namespace wjq

@@ -15,9 +15,10 @@
 //               resolution, the filter, and either the aggregate or a
 //               compact record per selected row (line offset, row length,
 //               field spans).
-//   k_rows_*    Rows only: block sums and an exclusive prefix over the
-//               per-tile (rows, bytes, lines) totals, then the rows are
-//               copied in line order from the input to the output.
+//   k_tail      Group results, the exclusive prefix over the tiles' (rows,
+//               bytes, lines) totals, first bad lines and FP totals.
+//   k_rows_emit Rows only: copies them in line order from the input to the
+//               output.
 //
 // No host synchronisation happens inside a run and no kernel waits on
 // another CTA.
@@ -26,6 +27,8 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "../../include/warpjq_ext.h"
 #include "../../include/warpjq_kernels.h"
@@ -38,7 +41,6 @@ namespace wjq {
 
 constexpr int kThreads = 32;                 // one warp per CTA; each warp owns its tile
 constexpr uint32_t kMaxLinesPerPass = 128;   // line-start list capacity per pass
-constexpr int kReduceThreads = 128;          // block size of the per-tile reductions
 // Register budgets of k_scan (CTAs of one warp per SM), measured per variant
 // on 1 GB of the nginx workload: the ungrouped aggregate at 20 (96 registers,
 // 8 bytes of spills: 685 us; at 24, with 144 bytes, 713; at 16, 775), the row
@@ -1488,66 +1490,11 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
   flush_counts(sp.ctr, nullptr, P, kRows, lane, acc, cta_fix);
 }
 
-// The index of the first invalid / type-error line: lines of the tiles
-// before the first tile holding one, summed in two passes (contiguous blocks
-// of tiles, then one warp over the block sums).
-__global__ void k_reduce_tiles(unsigned long long n_tiles, const TileDesc *tiles, RunCounters *ctr,
-                               unsigned long long *block_lines) {
-  __shared__ unsigned long long s_l[kReduceThreads], s_t[kReduceThreads];
-  unsigned long long per = (n_tiles + gridDim.x - 1) / gridDim.x;
-  unsigned long long b0 = blockIdx.x * per, b1 = min(b0 + per, n_tiles);
-  unsigned long long cut = ctr->first_invalid_tile, cut_t = ctr->first_type_tile;
-  unsigned long long lines = 0, lines_t = 0;
-  unsigned long long chunk = (b1 > b0 ? b1 - b0 : 0);
-  unsigned long long cper = (chunk + kReduceThreads - 1) / kReduceThreads;
-  unsigned long long c0 = b0 + threadIdx.x * cper, c1 = min(c0 + cper, b1);
-  for (unsigned long long t = c0; t < c1 && (t < cut || t < cut_t); t++) {
-    if (t < cut) lines += tiles[t].n_lines;
-    if (t < cut_t) lines_t += tiles[t].n_lines;
-  }
-  s_l[threadIdx.x] = lines;
-  s_t[threadIdx.x] = lines_t;
-  __syncthreads();
-  for (int d = kReduceThreads / 2; d > 0; d >>= 1) {
-    if (threadIdx.x < d) {
-      s_l[threadIdx.x] += s_l[threadIdx.x + d];
-      s_t[threadIdx.x] += s_t[threadIdx.x + d];
-    }
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    block_lines[2 * blockIdx.x] = s_l[0];
-    block_lines[2 * blockIdx.x + 1] = s_t[0];
-  }
-}
-
 // The run's FP totals from its exact limbs (the integer sum joins them
 // before the one rounding of sum_total).
 __device__ __forceinline__ void finalize_sums(RunCounters &c) {
   c.fsum_total = fix_to_double(c.fix, 0, 0) + c.fbig;
   c.sum_total = fix_to_double(c.fix, c.agg_isum_lo, c.agg_isum_hi) + c.fbig;
-}
-
-// One warp: the block sums of k_reduce_tiles, then the first bad lines and
-// the FP totals.
-__global__ void k_finalize(const unsigned long long *block_lines, unsigned nblocks, const TileDesc *tiles,
-                           RunCounters *ctr) {
-  const int lane = threadIdx.x;
-  unsigned long long lines = 0, lines_t = 0;
-  for (unsigned b = lane; b < nblocks; b += 32) {
-    lines += block_lines[2 * b];
-    lines_t += block_lines[2 * b + 1];
-  }
-#pragma unroll
-  for (int d = 16; d > 0; d >>= 1) {
-    lines += __shfl_down_sync(0xffffffffu, lines, d);
-    lines_t += __shfl_down_sync(0xffffffffu, lines_t, d);
-  }
-  if (lane != 0) return;
-  finalize_sums(*ctr);
-  unsigned long long cut = ctr->first_invalid_tile, cut_t = ctr->first_type_tile;
-  ctr->first_invalid = cut == ~0ull ? ~0ull : lines + tiles[cut].first_invalid;
-  ctr->first_type_error = cut_t == ~0ull ? ~0ull : lines_t + tiles[cut_t].first_type_error;
 }
 
 // The keys that hold lines (not the ids that inserts racing for a key left
@@ -1556,9 +1503,8 @@ __global__ void k_finalize(const unsigned long long *block_lines, unsigned nbloc
 // Compacting and rounding them here leaves the host one copy of 88 bytes a
 // group: 60 ns a group before (the raw descriptors and accumulators of every
 // id, 152 bytes each, through pageable memory, then two roundings).
-__global__ void __launch_bounds__(256) k_groups_compact(RunCounters *ctr, const GroupKeyDesc *keys,
-                                                        const GroupAcc *acc, uint32_t key_cap,
-                                                        warpjq_group_ext *out, uint32_t *out_input) {
+__device__ __forceinline__ void compact_groups(RunCounters *ctr, const GroupKeyDesc *keys, const GroupAcc *acc,
+                                               uint32_t key_cap, warpjq_group_ext *out, uint32_t *out_input) {
   const uint32_t nk = min(ctr->n_keys, key_cap);
   for (uint32_t k0 = blockIdx.x * blockDim.x; k0 < nk; k0 += gridDim.x * blockDim.x) {
     const uint32_t k = k0 + threadIdx.x;
@@ -1680,8 +1626,6 @@ constexpr int kEmitThreads = 128;
 __host__ __device__ inline uint32_t rows_tiles_per_block(unsigned long long n_tiles) {
   return n_tiles < 148ull * 8 ? 8u : n_tiles < 262144ull ? 64u : 128u;
 }
-constexpr int kPrefixThreads = 1024;  // the one block that scans the block sums
-
 // Exclusive block scan of three u64 values in thread order, with totals.
 template <int NT>
 __device__ __forceinline__ void block_scan3(const unsigned long long v[3], unsigned long long ex[3],
@@ -1712,54 +1656,102 @@ __device__ __forceinline__ void block_scan3(const unsigned long long v[3], unsig
   __syncthreads();
 }
 
-// Pass 1: (rows, bytes, lines) summed per block of `tpb` tiles.
-__global__ void __launch_bounds__(kEmitThreads)
-    k_rows_block_sums(const RowTile *rt, const TileDesc *td, unsigned long long n_tiles,
-                      uint32_t tpb, unsigned long long *bsum) {
-  __shared__ unsigned long long s_w[3][kEmitThreads / 32];
-  const unsigned long long t0 = (unsigned long long)blockIdx.x * tpb;
-  unsigned long long v[3] = {0, 0, 0};
-  const unsigned long long t = t0 + threadIdx.x;
-  if (threadIdx.x < tpb && t < n_tiles) {
-    v[0] = rt[t].rows;
-    v[1] = rt[t].bytes;
-    v[2] = td[t].n_lines;
-  }
-  unsigned long long ex[3], tot[3];
-  block_scan3<kEmitThreads>(v, ex, tot, s_w);
-  if (threadIdx.x == 0)
-    for (int k = 0; k < 3; k++) bsum[blockIdx.x * 3 + k] = tot[k];
-}
+// The run's last pass over its tiles, in blocks of `tpb` of them: the group
+// results, sums of (rows, bytes, lines) per block, and in the block that is
+// through last everything that needs them all: for rows the exclusive prefix
+// over the blocks (in place; output that does not fit raises the overflow
+// flag, and the run is repeated with room), the indexes of the first invalid
+// and type-error line, and the FP totals.  One launch where the same took four
+// (two without rows): a run of 4 KB spent 9 of its 23 us on the device there.
+struct TailParams {
+  unsigned long long n_tiles;
+  uint32_t tpb;
+  const TileDesc *tiles;
+  const RowTile *row_tiles;  // null: no rows
+  unsigned long long *bsum;  // 3 per block
+  RunCounters *ctr;
+  unsigned long long *row_off;
+  unsigned long long rows_cap, out_cap;
+  const GroupKeyDesc *keys;  // null: no groups
+  const GroupAcc *acc;
+  uint32_t key_cap;
+  warpjq_group_ext *ext;
+  uint32_t *ext_input;
+};
+constexpr int kTailThreads = 256;
+constexpr unsigned kTailBlocks = 256;  // of a run without rows, at most
 
-// Pass 2 (one block): block sums -> exclusive block prefixes, in place; the
-// totals give the output length and the closing row offset.  Output that
-// does not fit raises the overflow flag (the run is repeated with room).
-__global__ void __launch_bounds__(kPrefixThreads)
-    k_rows_block_prefix(unsigned long long *bsum, unsigned nblocks, RunCounters *ctr,
-                        unsigned long long *row_off, unsigned long long rows_cap,
-                        unsigned long long out_cap) {
-  __shared__ unsigned long long s_w[3][kPrefixThreads / 32];
-  const unsigned per = (nblocks + kPrefixThreads - 1) / kPrefixThreads;
-  const unsigned b0 = threadIdx.x * per, b1 = min(b0 + per, nblocks);
-  unsigned long long v[3] = {0, 0, 0};
-  for (unsigned b = b0; b < b1; b++)
-    for (int k = 0; k < 3; k++) v[k] += bsum[b * 3 + k];
-  unsigned long long ex[3], tot[3];
-  block_scan3<kPrefixThreads>(v, ex, tot, s_w);
-  for (unsigned b = b0; b < b1; b++)
-    for (int k = 0; k < 3; k++) {
-      unsigned long long x = bsum[b * 3 + k];
-      bsum[b * 3 + k] = ex[k];
-      ex[k] += x;
+__global__ void __launch_bounds__(kTailThreads) k_tail(const __grid_constant__ TailParams tp) {
+  __shared__ unsigned long long s_w[3][kTailThreads / 32];
+  __shared__ uint32_t s_last;
+  RunCounters &c = *tp.ctr;
+  if (tp.keys) compact_groups(tp.ctr, tp.keys, tp.acc, tp.key_cap, tp.ext, tp.ext_input);
+  const unsigned long long cut[2] = {c.first_invalid_tile, c.first_type_tile};
+  const bool bad = cut[0] != ~0ull || cut[1] != ~0ull, sums = tp.row_tiles || bad;
+  unsigned long long v[3] = {0, 0, 0}, ex[3], tot[3];
+  if (sums) {
+    const unsigned long long t0 = (unsigned long long)blockIdx.x * tp.tpb, t1 = min(t0 + tp.tpb, tp.n_tiles);
+    for (unsigned long long t = t0 + threadIdx.x; t < t1; t += kTailThreads) {
+      if (tp.row_tiles) {
+        v[0] += tp.row_tiles[t].rows;
+        v[1] += tp.row_tiles[t].bytes;
+      }
+      v[2] += tp.tiles[t].n_lines;
     }
-  if (threadIdx.x == 0) {
-    ctr->out_len = tot[1];
-    if (tot[0] > rows_cap || tot[1] > out_cap) atomicOr(&ctr->overflow, 2u);
-    else row_off[tot[0]] = tot[1];
+    block_scan3<kTailThreads>(v, ex, tot, s_w);
   }
+  if (threadIdx.x == 0) {
+    if (sums)
+      for (int k = 0; k < 3; k++) tp.bsum[blockIdx.x * 3 + k] = tot[k];
+    __threadfence();
+    s_last = atomicAdd(&c.tail_done, 1u) + 1 == gridDim.x;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();  // the other blocks' sums are there
+  if (sums) {
+    const unsigned nb = gridDim.x, per = (nb + kTailThreads - 1) / kTailThreads;
+    const unsigned b0 = min(threadIdx.x * per, nb), b1 = min(b0 + per, nb);
+    v[0] = v[1] = v[2] = 0;
+    for (unsigned b = b0; b < b1; b++)
+      for (int k = 0; k < 3; k++) v[k] += __ldcg(tp.bsum + b * 3 + k);
+    block_scan3<kTailThreads>(v, ex, tot, s_w);
+    for (unsigned b = b0; b < b1; b++)
+      for (int k = 0; k < 3; k++) {
+        const unsigned long long x = __ldcg(tp.bsum + b * 3 + k);
+        tp.bsum[b * 3 + k] = ex[k];
+        ex[k] += x;
+      }
+    if (threadIdx.x == 0 && tp.row_tiles) {
+      c.out_len = tot[1];
+      if (tot[0] > tp.rows_cap || tot[1] > tp.out_cap) atomicOr(&c.overflow, 2u);
+      else tp.row_off[tot[0]] = tot[1];
+    }
+    __syncthreads();
+  }
+  if (bad) {  // lines before the first tile that holds one: of the blocks before its block, then of its tiles
+    v[0] = v[1] = v[2] = 0;
+    for (int k = 0; k < 2; k++)
+      if (cut[k] != ~0ull)
+        for (unsigned long long t = cut[k] / tp.tpb * tp.tpb + threadIdx.x; t < cut[k]; t += kTailThreads)
+          v[k] += tp.tiles[t].n_lines;
+    block_scan3<kTailThreads>(v, ex, tot, s_w);
+  }
+  if (threadIdx.x != 0) return;
+  finalize_sums(c);
+  c.first_invalid = cut[0] == ~0ull ? ~0ull : tp.bsum[cut[0] / tp.tpb * 3 + 2] + tot[0] + tp.tiles[cut[0]].first_invalid;
+  c.first_type_error =
+      cut[1] == ~0ull ? ~0ull : tp.bsum[cut[1] / tp.tpb * 3 + 2] + tot[1] + tp.tiles[cut[1]].first_type_error;
 }
 
-// Pass 3: each block takes its `tiles_per_block` tiles: per-tile prefixes by a
+// Tiles per block of k_tail, and its blocks.
+inline uint32_t tail_tiles_per_block(unsigned long long n_tiles, bool rows) {
+  return rows ? rows_tiles_per_block(n_tiles)
+              : (uint32_t)std::max<unsigned long long>(32, (n_tiles + kTailBlocks - 1) / kTailBlocks);
+}
+inline unsigned tail_blocks(unsigned long long n_tiles, uint32_t tpb) { return (unsigned)((n_tiles + tpb - 1) / tpb); }
+
+// The rows' copy: each block takes its `tiles_per_block` tiles: per-tile prefixes by a
 // block scan, then the block's rows, in order.  Whole lines are copied a row a
 // group of lanes.  Rows of values are short, so they take a thread each, which
 // puts its bytes into shared memory; the block then writes the batch's rows,

@@ -55,14 +55,13 @@ constexpr uint32_t kNoAllocHalo = 2048;
 constexpr uint64_t kNoAllocMaxTiles = kNoAllocMaxInput / kNoAllocTile;
 constexpr uint32_t kNoAllocMaxGrid = 2048;
 constexpr uint64_t kNoAllocDeepLevels = 1u << 14;  // per CTA, beyond the 64 in registers
-constexpr unsigned kNoAllocReduceBlocks = 256;
 
 constexpr uint64_t align256(uint64_t x) { return (x + 255) & ~255ull; }
 constexpr uint64_t kOffCtr = 0;
 constexpr uint64_t kOffTiles = align256(kOffCtr + sizeof(RunCounters));
 constexpr uint64_t kOffBlockLines = align256(kOffTiles + kNoAllocMaxTiles * sizeof(TileDesc));
 constexpr uint64_t kOffDeep =
-    align256(kOffBlockLines + 2 * kNoAllocReduceBlocks * sizeof(unsigned long long));
+    align256(kOffBlockLines + 3 * kTailBlocks * sizeof(unsigned long long));
 constexpr uint64_t kScratchBytes =
     align256(kOffDeep + kNoAllocMaxGrid * (kNoAllocDeepLevels / 32) * sizeof(uint32_t));
 
@@ -230,14 +229,15 @@ extern "C" warpjq_status warpjq_aggregate_noalloc(const warpjq_program *prog, co
       e = cudaLaunchKernel((const void *)k_scan<false>, dim3(grid), dim3(kThreads), args, s->smem, st);
     }
     if (e == cudaSuccess) {
-      unsigned nb = kNoAllocReduceBlocks;
-      void *args[] = {&n_tiles, &tiles, &ctr, &block_lines};
-      e = cudaLaunchKernel((const void *)k_reduce_tiles, dim3(nb), dim3(kReduceThreads), args, 0, st);
-    }
-    if (e == cudaSuccess) {
-      unsigned nb = kNoAllocReduceBlocks;
-      void *args[] = {&block_lines, &nb, &tiles, &ctr};
-      e = cudaLaunchKernel((const void *)k_finalize, dim3(1), dim3(32), args, 0, st);
+      TailParams tp;
+      memset(&tp, 0, sizeof(tp));
+      tp.n_tiles = n_tiles;
+      tp.tpb = tail_tiles_per_block(n_tiles, false);
+      tp.tiles = tiles;
+      tp.bsum = block_lines;
+      tp.ctr = ctr;
+      void *args[] = {&tp};
+      e = cudaLaunchKernel((const void *)k_tail, dim3(tail_blocks(n_tiles, tp.tpb)), dim3(kTailThreads), args, 0, st);
     }
   }
   if (e == cudaSuccess) {

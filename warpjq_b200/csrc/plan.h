@@ -127,7 +127,7 @@ struct RunCounters {
   unsigned int overflow;     // bit0 records, bit1 output, bit2 groups, bit3 deep stack
   unsigned int error;        // nonzero: a kernel found its own state inconsistent
   unsigned int n_groups;     // written by the group compaction: keys that hold lines
-  unsigned int pad;
+  unsigned int tail_done;    // blocks of the run's last pass that are through
   // exact sum of the non-integer aggregate values (fixsum.cuh): limb k
   // counts units of 2^(32 k - 128); values of magnitude >= 2^128 go to fbig
   long long fix[8];
