@@ -250,14 +250,14 @@ __host__ __device__ constexpr uint32_t csv_smem(bool write) { return kCsvOff + (
 // The hits of eight words: ',' '"' '\\' and bytes below 0x20 (devutil.cuh
 // flags_special, with ',').
 __device__ __forceinline__ uint32_t csv_hits(const uint32_t w[8]) {
-  uint32_t m = 0;
+  uint32_t f[8];
 #pragma unroll
-  for (int k = 7; k >= 0; k--) {
+  for (int k = 0; k < 8; k++) {
     const uint32_t t = (w[k] ^ 0x02020202u) & 0x7F7F7F7Fu;
     const uint32_t sq = t + 0x5F5F5F5Fu, sb = (t ^ 0x5E5E5E5Eu) + 0x7F7F7F7Fu, sc = (t ^ 0x2E2E2E2Eu) + 0x7F7F7F7Fu;
-    m = wjq::flags_push(m, ~((sq & sb & sc) | w[k]) & 0x80808080u);
+    f[k] = ~((sq & sb & sc) | w[k]) & 0x80808080u;
   }
-  return m;
+  return wjq::flags_gather(f);
 }
 
 // Output into shared memory from byte `at` on, a word at a time; the words a

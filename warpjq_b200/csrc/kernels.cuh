@@ -952,8 +952,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
     const uint32_t nl_limit = tlen - 1;  // newlines below this start a line in the tile
     // the newlines of chunk c that start a line of the tile
     auto listed = [&](uint32_t c, uint32_t m) -> uint32_t {
-      const uint32_t left = c * 32 < nl_limit ? nl_limit - c * 32 : 0u;
-      return left >= 32 ? m : m & ((1u << left) - 1u);
+      const int left = max((int)nl_limit - (int)(c * 32), 0);
+      return m & ~__funnelshift_lc(0u, 0xFFFFFFFFu, (uint32_t)left);  // all bits from 32 on
     };
     uint32_t my_nl = 0;
     unsigned long long nl_pos = 0;  // positions within the lane's chunks, 8 bits each
@@ -966,9 +966,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       uint32_t sm_c;
       uint32_t m = listed(c, classify_chunk(w8, &sm_c));
       smask[c] = sm_c;
-      my_nl += __popc(m);
 #pragma unroll 1
-      for (; m; m &= m - 1u) nl_pos = nl_pos << 8 | ((c - c0) * 32u + (uint32_t)__ffs(m) - 1u);
+      for (; m; m &= m - 1u, my_nl++) nl_pos = nl_pos << 8 | ((c - c0) * 32u + (uint32_t)__ffs(m) - 1u);
     }
 
     // The next tile's window is fetched into L2 now (its ticket has

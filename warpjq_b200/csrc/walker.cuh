@@ -1221,11 +1221,12 @@ __device__ __forceinline__ int walk_template(const Template *t, const uint8_t *w
   for (uint32_t j = 0; j < ns; j++) {
     const uint32_t d = t->desc[j];
     {
-      const uint32_t *q = (const uint32_t *)w + (p >> 2), *L = t->lit[j], *M = t->mask[j];
+      const uint32_t *q = (const uint32_t *)w + (p >> 2);
+      const uint4 L = *(const uint4 *)t->lit[j], M = *(const uint4 *)t->mask[j];
       const uint32_t sh = (p & 3u) * 8u;
       const uint32_t a = q[0], b = q[1], c = q[2], f = q[3], g = q[4];
-      const uint32_t bad = ((__funnelshift_r(a, b, sh) ^ L[0]) & M[0]) | ((__funnelshift_r(b, c, sh) ^ L[1]) & M[1]) |
-                           ((__funnelshift_r(c, f, sh) ^ L[2]) & M[2]) | ((__funnelshift_r(f, g, sh) ^ L[3]) & M[3]);
+      const uint32_t bad = ((__funnelshift_r(a, b, sh) ^ L.x) & M.x) | ((__funnelshift_r(b, c, sh) ^ L.y) & M.y) |
+                           ((__funnelshift_r(c, f, sh) ^ L.z) & M.z) | ((__funnelshift_r(f, g, sh) ^ L.w) & M.w);
       // no literal holds a newline, so one that fits ends at or before e
       on = on && !bad;
       if (on) p += d & 0xFFu;
