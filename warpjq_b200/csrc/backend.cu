@@ -162,7 +162,8 @@ struct Slot {
   uint8_t *d_chunk = nullptr;
   unsigned long long n_bytes = 0;
   RunBufs rb;
-  RunCounters *h_ctr = nullptr;  // pinned mirror
+  RunCounters *h_ctr = nullptr;  // pinned mirror of the last run's counters
+  bool mirrored = false;         // the last run's kernels write it
   // pinned result mirrors
   std::vector<uint8_t> dummy;
   uint8_t *h_out = nullptr;
@@ -423,6 +424,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     CK(cudaEventRecord(s.btab_done, st), "event record");
   }
   s.kernels = 0;
+  s.mirrored = n > 0 && n_tiles > 0;
   if (b && n_inputs) {
     k_batch_reset<<<(n_inputs + 255) / 256, 256, 0, st>>>(rb.b_in_ctr.p, n_inputs);
     s.kernels++;
@@ -529,6 +531,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     tp.row_tiles = rows ? rb.row_tiles.p : nullptr;
     tp.bsum = rb.row_bsum.p;
     tp.ctr = rb.ctr.p;
+    tp.mirror = s.h_ctr;
     tp.row_off = rb.row_off.p;
     tp.rows_cap = rb.rows_cap;
     tp.out_cap = rb.out_cap;
@@ -650,8 +653,8 @@ warpjq_status run_to_completion(warpjq_ctx *c, Slot &s, const uint8_t *d_data,
       warpjq_status rc = enqueue_run(c, s, d_data, n, st, err, err_len, b);
       if (rc != WARPJQ_OK) return rc;
     }
-    CK(cudaMemcpyAsync(s.h_ctr, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st),
-       "D2H counters");
+    if (!s.mirrored)
+      CK(cudaMemcpyAsync(s.h_ctr, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st), "D2H counters");
     if (run_grouped(c, b)) {  // few groups come along, without a second wait
       warpjq_status rc = ensure_host_groups(s, kFirstGroups, err, err_len);
       if (rc != WARPJQ_OK) return rc;
@@ -1389,6 +1392,7 @@ struct warpjq_batch_graph {
   std::vector<warpjq_ctx *> ctxs;
   std::vector<uint64_t> epochs, sigs;
   std::vector<uint32_t> kernels;
+  std::vector<bool> mirrored;  // Slot::mirrored of each batch
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 };
@@ -1458,6 +1462,7 @@ warpjq_status warpjq_batch_graph_create(warpjq_ctx *const *ctxs, uint32_t n_ctx,
     rc = enqueue_run(c, c->dev, c->batch.d_data, c->batch.total, ss[i], err, err_len, &c->batch);
     c->batch.tables_on_device = false;
     g->kernels.push_back(c->dev.kernels);
+    g->mirrored.push_back(c->dev.mirrored);
     if (rc != WARPJQ_OK) break;
     if ((e = cudaEventRecord(joins[i], ss[i])) != cudaSuccess) fail(e, "capture join");
     else if ((e = cudaStreamWaitEvent(s0, joins[i], 0)) != cudaSuccess) fail(e, "capture join");
@@ -1511,6 +1516,7 @@ warpjq_status warpjq_batch_graph_launch(warpjq_batch_graph *g, void *stream, cha
     c->batch.active = true;
     c->batch.stream = st;
     c->dev.launched = true;
+    c->dev.mirrored = g->mirrored[i];
     c->dev.timed = false;
     c->dev.kernels = g->kernels[i];
   }

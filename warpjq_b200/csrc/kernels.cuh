@@ -1669,6 +1669,7 @@ struct TailParams {
   const RowTile *row_tiles;  // null: no rows
   unsigned long long *bsum;  // 3 per block
   RunCounters *ctr;
+  RunCounters *mirror;  // page-locked host memory that gets the finished counters (null: none)
   unsigned long long *row_off;
   unsigned long long rows_cap, out_cap;
   const GroupKeyDesc *keys;  // null: no groups
@@ -1736,11 +1737,19 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(const __grid_constant__ T
           v[k] += tp.tiles[t].n_lines;
     block_scan3<kTailThreads>(v, ex, tot, s_w);
   }
-  if (threadIdx.x != 0) return;
-  finalize_sums(c);
-  c.first_invalid = cut[0] == ~0ull ? ~0ull : tp.bsum[cut[0] / tp.tpb * 3 + 2] + tot[0] + tp.tiles[cut[0]].first_invalid;
-  c.first_type_error =
-      cut[1] == ~0ull ? ~0ull : tp.bsum[cut[1] / tp.tpb * 3 + 2] + tot[1] + tp.tiles[cut[1]].first_type_error;
+  if (threadIdx.x == 0) {
+    finalize_sums(c);
+    c.first_invalid = cut[0] == ~0ull ? ~0ull : tp.bsum[cut[0] / tp.tpb * 3 + 2] + tot[0] + tp.tiles[cut[0]].first_invalid;
+    c.first_type_error =
+        cut[1] == ~0ull ? ~0ull : tp.bsum[cut[1] / tp.tpb * 3 + 2] + tot[1] + tp.tiles[cut[1]].first_type_error;
+    __threadfence();
+  }
+  // The host reads the counters once the stream is done, with no copy of its
+  // own behind the kernel (5 us of a 4 KB run).
+  __syncthreads();
+  static_assert(sizeof(RunCounters) % 8 == 0, "copied by words");
+  if (tp.mirror && threadIdx.x < sizeof(RunCounters) / 8)
+    ((unsigned long long *)tp.mirror)[threadIdx.x] = __ldcg((const unsigned long long *)tp.ctr + threadIdx.x);
 }
 
 // Tiles per block of k_tail, and its blocks.
