@@ -33,7 +33,7 @@ enum LineStatus : int {
 // Values recorded per trie node for one line; offsets are relative to the
 // line start.
 struct NodeVals {
-  uint8_t kind[kMaxNodes];
+  alignas(4) uint8_t kind[kMaxNodes];
   uint8_t esc[kMaxNodes];
   uint32_t off[kMaxNodes];
   uint32_t len[kMaxNodes];
@@ -743,7 +743,8 @@ __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, con
   int status = LS_FALLBACK;
   on = on && w[s] == '{';
 #pragma unroll 1
-  for (uint32_t k = 0; k < n_nodes; k++) v.kind[k] = JK_MISSING;
+  for (uint32_t k = 0; k < n_nodes; k += 4) *(uint32_t *)(v.kind + k) = 0;  // JK_MISSING, four nodes a store
+  unsigned long long seen = 1;  // nodes a value has landed on
   uint32_t cur = n_nodes ? 0u : kNoNode;  // trie node of the innermost open object
   unsigned long long lm = 0;             // its key_len_mask (0: no key is looked up)
   if (cur != kNoNode) {
@@ -783,8 +784,11 @@ __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, con
     }
     warp_meet();
     if (on && vn != kNoNode) {
+      // a key that comes again replaces what its first value held below it
+      if ((seen >> vn) & 1ull)
 #pragma unroll 1
-      for (uint32_t x = vn + 1u; x < P.nodes[vn].subtree_end; x++) v.kind[x] = JK_MISSING;
+        for (uint32_t x = vn + 1u; x < P.nodes[vn].subtree_end; x++) v.kind[x] = JK_MISSING;
+      seen |= 1ull << vn;
       v.kind[vn] = kind_of(c);
       v.off[vn] = vs - s;
       v.esc[vn] = 0;
