@@ -45,23 +45,6 @@ __device__ __forceinline__ uint32_t swar_string_special(uint32_t x) {
   return (zq | zb | lo) & 0x80808080u;
 }
 
-// SWAR: nonzero iff some byte of `x` is '\n'.
-__device__ __forceinline__ uint32_t swar_newline(uint32_t x) {
-  uint32_t t = x ^ 0x0A0A0A0Au;
-  return (t - 0x01010101u) & ~t & 0x80808080u;
-}
-
-// Exact per-byte newline flags: 0x80 in each byte lane holding '\n'.
-__device__ __forceinline__ uint32_t swar_newline_exact(uint32_t x) {
-  uint32_t t = x ^ 0x0A0A0A0Au;
-  return ~(((t & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | t) & 0x80808080u;
-}
-
-// Gathers the four 0x80 flags of `m` into bits 0..3.
-__device__ __forceinline__ uint32_t swar_movemask(uint32_t m) {
-  return ((m >> 7) * 0x00204081u) >> 21 & 0xFu;
-}
-
 // ---------------------------------------------------------------------------
 // Structural classification of 32-byte chunks (the scan's first stage)
 // ---------------------------------------------------------------------------

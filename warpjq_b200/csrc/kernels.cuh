@@ -170,7 +170,9 @@ static_assert(sizeof(GroupKeyDesc) == 24, "group key descriptor");
 // Most rounds are counts, extremes and sums of plain integers: those go by
 // 32-bit shared atomics into n, num, lo and hi (a sum's values as two halves;
 // for extremes, lo counts the integers), which hold kFoldLines lines before
-// they are folded into the accumulators.
+// they are folded into the accumulators.  (group_by(.path) | count over 500 MB,
+// 32 keys: 546 us; with accumulators for 16 key ids and every round's keys
+// looked up in the table, 675.)
 constexpr uint32_t kKeyCache = 32;       // one lane clears one
 constexpr uint32_t kKeyCacheBytes = 24;  // longest key kept
 constexpr uint32_t kKeyAccBytes = 2048;
@@ -1500,7 +1502,7 @@ __device__ __forceinline__ void finalize_sums(RunCounters &c) {
 // unused), as the results the host hands on: exact sums rounded once
 // (fixsum.cuh), minima and maxima decoded.  Their order is any, like the ids'.
 // Compacting and rounding them here leaves the host one copy of 88 bytes a
-// group: 60 ns a group before (the raw descriptors and accumulators of every
+// group: some 160 ns a group before (the raw descriptors and accumulators of every
 // id, 152 bytes each, through pageable memory, then two roundings).
 __device__ __forceinline__ void compact_groups(RunCounters *ctr, const GroupKeyDesc *keys, const GroupAcc *acc,
                                                uint32_t key_cap, warpjq_group_ext *out, uint32_t *out_input) {
