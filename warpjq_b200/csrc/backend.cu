@@ -627,6 +627,7 @@ bool grow_after_overflow(warpjq_ctx *c, Slot &s, const RunCounters &h, unsigned 
 }
 
 constexpr size_t kFirstGroups = 64;          // copied with the counters
+constexpr size_t kHostGroups = 8192;         // first page-locked room (0.7 MB), taken with a grouped context
 constexpr size_t kPinnedGroups = 1u << 20;  // page-locked room for results grows up to this (92 MB)
 
 warpjq_status ensure_host_groups(Slot &s, size_t n, char *err, size_t err_len) {
@@ -636,7 +637,9 @@ warpjq_status ensure_host_groups(Slot &s, size_t n, char *err, size_t err_len) {
   s.h_ext = nullptr;
   s.h_in = nullptr;
   s.h_ext_cap = 0;
-  const size_t cap = std::max(n, std::min(n + n / 4, kPinnedGroups));
+  // Page-locking and releasing memory stalls the whole device, so a slot does
+  // it seldom: from kHostGroups on, at least doubling.
+  const size_t cap = std::max(n, std::min(std::max(2 * n, kHostGroups), kPinnedGroups));
   CK(cudaHostAlloc((void **)&s.h_ext, cap * sizeof(warpjq_group_ext), cudaHostAllocDefault), "pinned groups");
   CK(cudaHostAlloc((void **)&s.h_in, cap * sizeof(uint32_t), cudaHostAllocDefault), "pinned groups");
   s.h_ext_cap = cap;
@@ -801,6 +804,10 @@ warpjq_status warpjq_ctx_create(const warpjq_program *prog, uint64_t max_chunk_b
     }
   }
   CK(cudaHostAlloc((void **)&c->dev.h_ctr, sizeof(RunCounters), cudaHostAllocDefault), "pinned ctr");
+  if (run_grouped(c.get(), nullptr)) {
+    rc = ensure_host_groups(c->dev, kHostGroups, err, err_len);
+    if (rc != WARPJQ_OK) return rc;
+  }
   *out = c.release();
   return WARPJQ_OK;
 }
