@@ -1687,7 +1687,10 @@ __global__ void __launch_bounds__(kTailThreads) k_tail(const __grid_constant__ T
   __shared__ unsigned long long s_w[3][kTailThreads / 32];
   __shared__ uint32_t s_last;
   RunCounters &c = *tp.ctr;
-  if (tp.keys) compact_groups(tp.ctr, tp.keys, tp.acc, tp.key_cap, tp.ext, tp.ext_input);
+  if (tp.keys) {
+    compact_groups(tp.ctr, tp.keys, tp.acc, tp.key_cap, tp.ext, tp.ext_input);
+    __syncthreads();  // all of the block's groups are counted before thread 0 says that it is through
+  }
   const unsigned long long cut[2] = {c.first_invalid_tile, c.first_type_tile};
   const bool bad = cut[0] != ~0ull || cut[1] != ~0ull, sums = tp.row_tiles || bad;
   unsigned long long v[3] = {0, 0, 0}, ex[3], tot[3];
