@@ -1102,8 +1102,10 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
         // Everything below, to the next bracket, is for lines no template fits.
         if (__any_sync(0xffffffffu, walk || (li < cnt && !found))) {
           const bool far = li < cnt && !found;
-          const int st = walk_objects(P, win, smask, s, e, nv, walk);  // every lane
-          if (walk) status = st == LS_FALLBACK ? walk_masked(P, win, smask, s, e, nv) : st;
+          if (walk) {
+            status = walk_objects(P, win, smask, s, e, nv);
+            if (status == LS_FALLBACK) status = walk_masked(P, win, smask, s, e, nv);
+          }
           if (far) {
             // longer than the window: walk it from global memory
             unsigned long long q = ts + wlen;

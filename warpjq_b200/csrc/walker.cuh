@@ -730,18 +730,18 @@ __device__ __forceinline__ bool warp_any(bool x) {
 // walk_masked costs its warp a walk of its own, so malformed lines are worth
 // deciding here.)  Same window contract as walk_masked.
 //
-// All lanes of a warp call it together, `on` where the lane has a line, and
-// take one member a turn: its key, then its value by kind, then the closing
-// brackets after it, meeting again after each (no lane leaves a turn early:
-// the compiler then runs the ones that stay apart from each other).  256 MB
-// of lines whose members come in different orders, 2% of them malformed, scan
-// in 902 us this way, against 1,077 when each lane ran on by itself.
+// Each lane walks its own line and leaves as soon as its verdict is known.  What
+// bounds it is instructions.  (Taking one member a turn with the warp together,
+// meeting after its key and after its value, cost a quarter more of them on
+// lines of one member order: scan of 192 MB of lines of 24 members, too long
+// for a template, 384 us that way and 292 so; of two interleaved shapes 286 and
+// 259; with an array each 471 and 431; 256 MB of members in any order, 2% of
+// the lines malformed, 897 and 903.)
 __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, const uint32_t *sm, uint32_t s,
-                                         uint32_t e, NodeVals &v, bool on = true) {
+                                         uint32_t e, NodeVals &v) {
   using namespace detail;
+  if (w[s] != '{') return LS_FALLBACK;
   const uint32_t n_nodes = P.n_nodes;
-  int status = LS_FALLBACK;
-  on = on && w[s] == '{';
 #pragma unroll 1
   for (uint32_t k = 0; k < n_nodes; k += 4) *(uint32_t *)(v.kind + k) = 0;  // JK_MISSING, four nodes a store
   unsigned long long seen = 1;  // nodes a value has landed on
@@ -756,34 +756,20 @@ __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, con
   unsigned long long stack = 0;  // trie nodes of the enclosing objects, 8 bits a level
   uint32_t depth = 1;
   uint32_t p = s + 1;  // where the next key's opening quote must be
-  bool opened = true;  // just after a '{'
-  // a byte that cannot be here, unless it is whitespace: the line's verdict
-  auto broken = [&](uint32_t x) {
-    on = false;
-    if (!is_ws3(x)) status = LS_INVALID;
-  };
-  while (warp_any(on)) {
-    uint32_t vn = kNoNode, vs = 0, c = 0;
-    if (on && w[p] != '"') {
-      if (opened && w[p] == '}') on = false;
-      else broken(w[p]);
-    }
-    if (on) {
-      const uint32_t q = next_special(sm, p + 1);
-      const uint32_t la = load4(w, q + 1);
-      if (w[q] != '"') {  // an escape, or a byte below 0x20 (the newline among them)
-        on = false;
-        if (w[q] != '\\') status = LS_INVALID;
-      } else if ((la & 0xFFu) != ':') {
-        broken(la & 0xFFu);
-      }
-      vs = q + 2;
-      c = (la >> 8) & 0xFFu;
-      const uint32_t kl = q - p - 1;
-      if (on && ((lm >> (kl < 63u ? kl : 63u)) & 1ull)) vn = match_key_win(P, (uint8_t)cur, w, p + 1, kl, false);
-    }
-    warp_meet();
-    if (on && vn != kNoNode) {
+  if (w[p] == '}') return LS_FALLBACK;
+#pragma unroll 1
+  for (;;) {
+    if (w[p] != '"') return is_ws3(w[p]) ? LS_FALLBACK : LS_INVALID;
+    const uint32_t q = next_special(sm, p + 1);
+    const uint32_t la = load4(w, q + 1);
+    if (w[q] != '"') return w[q] == '\\' ? LS_FALLBACK : LS_INVALID;
+    if ((la & 0xFFu) != ':') return is_ws3(la & 0xFFu) ? LS_FALLBACK : LS_INVALID;
+    const uint32_t vs = q + 2;
+    const uint32_t c = (la >> 8) & 0xFFu;
+    const uint32_t kl = q - p - 1;
+    uint32_t vn = kNoNode;
+    if ((lm >> (kl < 63u ? kl : 63u)) & 1ull) vn = match_key_win(P, (uint8_t)cur, w, p + 1, kl, false);
+    if (vn != kNoNode) {
       // a key that comes again replaces what its first value held below it
       if ((seen >> vn) & 1ull)
 #pragma unroll 1
@@ -793,78 +779,54 @@ __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, con
       v.off[vn] = vs - s;
       v.esc[vn] = 0;
     }
-    uint32_t ve = 0;  // the value's end; 0 when an object was opened
-    bool go = on && c == '"', esc = false;
-    if (go) {
+    uint32_t ve;
+    if (c == '"') {
       ve = vs + 1;
+      bool esc = false;
 #pragma unroll 1
-      while (go) {
-        const uint32_t k = ve >> 5, m = __funnelshift_r(sm[k], sm[k + 1], ve & 31u);
-        if (!m) {
-          ve += 32;
-        } else {
-          ve += (uint32_t)__ffs(m) - 1u;
-          const uint32_t x = w[ve];
-          go = x == '\\';
-          if (go) {
-            const uint32_t y = w[ve + 1];
-            esc = true;
-            if (!simple_escape(y)) on = go = y == 'u' && hex4_at(w, ve + 2);
-            ve++;
-          } else {
-            on = x == '"';
-          }
-          ve++;
-        }
+      for (;;) {
+        ve = next_special(sm, ve);
+        const uint32_t x = w[ve];
+        if (x == '"') break;
+        if (x != '\\') return LS_INVALID;  // a control byte, the newline among them
+        const uint32_t y = w[ve + 1];
+        esc = true;
+        if (!simple_escape(y) && !(y == 'u' && hex4_at(w, ve + 2))) return LS_INVALID;
+        ve += 2;
       }
-      if (!on) status = LS_INVALID;  // a control byte (the newline among them) or a bad escape
-      if (on && esc && vn != kNoNode) v.esc[vn] = 1;
+      ve++;
+      if (esc && vn != kNoNode) v.esc[vn] = 1;
+    } else if (c == '{') {
+      if (depth >= 8 || w[vs + 1] == '}') return LS_FALLBACK;
+      stack = (stack << 8) | cur;
+      depth++;
+      cur = vn;
+      lm = vn != kNoNode ? P.nodes[vn].key_len_mask : 0ull;
+      p = vs + 1;
+      continue;
+    } else {
+      if (c == '[') return LS_FALLBACK;
+      ve = win_atom(w, vs, c);
+      if (!ve) return is_ws3(c) ? LS_FALLBACK : LS_INVALID;
     }
-    warp_meet();
-    if (on && c != '"') {
-      if (c == '{') {
-        on = depth < 8;
-        stack = (stack << 8) | cur;
-        depth++;
-        cur = vn;
-        lm = vn != kNoNode ? P.nodes[vn].key_len_mask : 0ull;
-        p = vs + 1;
-        opened = true;
-      } else if (c == '[') {
-        on = false;
-      } else {
-        ve = win_atom(w, vs, c);
-        if (!ve) broken(c);
-      }
-    }
-    warp_meet();
-    if (on && ve) {
-      if (vn != kNoNode) v.len[vn] = ve - vs;
-      // after a value: ',' and the next key, or '}' closing one or more objects
-      uint32_t t = w[ve];
+    if (vn != kNoNode) v.len[vn] = ve - vs;
+    // after a value: ',' and the next key, or '}' closing one or more objects
+    uint32_t t = w[ve];
+    if (t == '}') {
 #pragma unroll 1
-      while (t == '}') {
+      do {
         ve++;
         if (cur != kNoNode) v.len[cur] = ve - s - v.off[cur];
-        depth--;
+        if (--depth == 0) return ve == e ? LS_OK : is_ws3(w[ve]) ? LS_FALLBACK : LS_INVALID;
         cur = (uint32_t)(stack & 0xFFu);
         stack >>= 8;
-        t = depth ? w[ve] : 0u;
-      }
-      if (!depth) {
-        on = false;
-        if (ve == e) status = LS_OK;
-        else if (!is_ws3(w[ve])) status = LS_INVALID;
-      } else if (t != ',') {
-        broken(t);
-      }
-      p = ve + 1;
-      opened = false;
-      lm = on && cur != kNoNode ? P.nodes[cur].key_len_mask : 0ull;
+        t = w[ve];
+      } while (t == '}');
+      lm = cur != kNoNode ? P.nodes[cur].key_len_mask : 0ull;
     }
-    warp_meet();
+    if (t != ',') return is_ws3(t) ? LS_FALLBACK : LS_INVALID;
+    p = ve + 1;
   }
-  return status;
 }
 
 // ---------------------------------------------------------------------------
