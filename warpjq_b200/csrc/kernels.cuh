@@ -944,8 +944,11 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
     // 2. Stage 1, lane-parallel: every 32-byte chunk of the window (the end
     //    sentinel's too) becomes its special mask; lane l owns chunks
     //    [l*K, l*K + K) and notes the newlines among them that start a line of
-    //    the tile, up to eight positions in one word each (the last ones
-    //    found lowest).  Bytes past the window's data are stale: no walk gets
+    //    the tile in one 64-bit word (the last ones found lowest): eight
+    //    positions of 8 bits, or, where a lane owns more than eight chunks
+    //    (the tiles of lines of 300 bytes and more), four of 16.  (With those
+    //    tiles' chunks classified again instead: lines of 1,000 bytes, 96 MB,
+    //    scan 88 us, 79 so.)  Bytes past the window's data are stale: no walk gets
     //    past its line's newline, so their mask bits are never looked at.
     const uint32_t limit = wlen + (win_reaches_end ? 1u : 0u);  // classified bytes
     const uint32_t nchunks = (limit + 31) >> 5;
@@ -958,7 +961,8 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       return m & ~__funnelshift_lc(0u, 0xFFFFFFFFu, (uint32_t)left);  // all bits from 32 on
     };
     uint32_t my_nl = 0;
-    unsigned long long nl_pos = 0;  // positions within the lane's chunks, 8 bits each
+    const uint32_t pos_bits = K <= 8 ? 8u : 16u;
+    unsigned long long nl_pos = 0;  // positions within the lane's chunks, pos_bits each
     const uint32_t c1 = min(c0 + K, nchunks);
 #pragma unroll 1
     for (uint32_t c = c0; c < c1; c++) {
@@ -969,7 +973,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
       uint32_t m = listed(c, classify_chunk(w8, &sm_c));
       smask[c] = sm_c;
 #pragma unroll 1
-      for (; m; m &= m - 1u, my_nl++) nl_pos = nl_pos << 8 | ((c - c0) * 32u + (uint32_t)__ffs(m) - 1u);
+      for (; m; m &= m - 1u, my_nl++) nl_pos = nl_pos << pos_bits | ((c - c0) * 32u + (uint32_t)__ffs(m) - 1u);
     }
 
     // The next tile's window is fetched into L2 now (its ticket has
@@ -1001,7 +1005,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
     const uint32_t lead = prev_nl;
     const uint32_t n_lines_tile = tot_nl + lead;
     // whether every lane's newlines are noted (else they are found again)
-    const bool noted = K <= 8 && !__any_sync(0xffffffffu, my_nl > 8);
+    const bool noted = !__any_sync(0xffffffffu, my_nl * pos_bits > 64u);
     // The tile's last line ends at the first newline at or after te - 1 (the
     // sentinel's, when the window reaches the data's end): looked for 512
     // bytes at a time, 16 a lane.
@@ -1036,7 +1040,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
 #pragma unroll 1
           for (uint32_t k = 0; k < my_nl; k++) {
             const uint32_t i = idx + my_nl - 1u - k - base;
-            if (i <= cnt) lstart[i] = (uint16_t)(c0 * 32u + ((uint32_t)(nl_pos >> (8 * k)) & 0xFFu) + 1u);
+            if (i <= cnt) lstart[i] = (uint16_t)(c0 * 32u + ((uint32_t)(nl_pos >> (pos_bits * k)) & ((1u << pos_bits) - 1u)) + 1u);
           }
         } else if (my_nl && idx <= base + cnt && idx + my_nl > base) {
           uint32_t i = idx - base;  // wraps below the pass

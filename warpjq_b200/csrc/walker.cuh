@@ -734,9 +734,8 @@ __device__ __forceinline__ bool warp_any(bool x) {
 // bounds it is instructions.  (Taking one member a turn with the warp together,
 // meeting after its key and after its value, cost a quarter more of them on
 // lines of one member order: scan of 192 MB of lines of 24 members, too long
-// for a template, 384 us that way and 292 so; of two interleaved shapes 286 and
-// 259; with an array each 471 and 431; 256 MB of members in any order, 2% of
-// the lines malformed, 897 and 903.)
+// for a template, 368 us that way and 275 so; of two interleaved shapes 286 and
+// 262; 256 MB of members in any order, 2% of the lines malformed, 883 and 882.)
 __device__ __noinline__ int walk_objects(const DevPlan &P, const uint8_t *w, const uint32_t *sm, uint32_t s,
                                          uint32_t e, NodeVals &v) {
   using namespace detail;
