@@ -154,8 +154,7 @@ struct GroupKeyDesc {
   uint32_t input;           // batch input the key belongs to (0 for one input)
   uint8_t kind;
   uint8_t esc;
-  uint8_t saw_non_numeric;  // a selected line had a non-numeric, non-null value
-  uint8_t pad[5];
+  uint8_t pad[6];
 };
 static_assert(sizeof(GroupKeyDesc) == 24, "group key descriptor");
 
@@ -1442,9 +1441,6 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
               if (frac) fix_atomic_add(a.fix, &a.fbig, fv);
             }
           }
-          if (kid != 0xFFFFFFFFu && !is_num && aggv.kind != JK_MISSING && aggv.kind != JK_NULL &&
-              P.agg_slot >= 0)
-            sp.g.keys[kid].saw_non_numeric = 1;
         }
 
         if (kRows) {
