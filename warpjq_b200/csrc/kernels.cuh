@@ -1441,6 +1441,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
               if (frac) fix_atomic_add(a.fix, &a.fbig, fv);
             }
           }
+          __syncwarp();  // kcache's keys and sums are there for the lanes that look in the next round
         }
 
         if (kRows) {
