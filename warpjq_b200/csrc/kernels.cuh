@@ -682,6 +682,33 @@ __device__ __forceinline__ void emit_row(const DevPlan &P, const uint8_t *line, 
   dst[w] = '\n';
 }
 
+// emit_row for JSON values and projections by a group of lanes (lane g of it).
+__device__ __forceinline__ void emit_row_group(const DevPlan &P, const uint8_t *line, const uint32_t *fields,
+                                               uint8_t *dst, uint32_t g) {
+  uint32_t w = 0;
+  auto text = [&](uint32_t at, uint32_t n) {  // of the plan's
+#pragma unroll 1
+    for (uint32_t k = g; k < n; k += kEmitLanes) dst[w + k] = P.blob[at + k];
+    w += n;
+  };
+  const bool proj = P.output_kind == 2;
+  const uint32_t nf = proj ? P.n_fields : 1;
+#pragma unroll 1
+  for (uint32_t f = 0; f < nf; f++) {
+    const uint32_t off = fields[2 * f], lk = fields[2 * f + 1], len = lk & 0x07FFFFFFu;
+    if (proj) text(P.prefix_off[f], P.prefix_len[f]);
+    if (lk >> 28 == JK_MISSING) {
+      if (g < 4) dst[w + g] = (uint8_t)(0x6C6C756Eu >> (8 * g));  // "null"
+      w += 4;
+    } else {
+      group_copy(dst + w, line + off, len, g);
+      w += len;
+    }
+  }
+  if (proj) text(P.suffix_off, P.suffix_len);
+  if (g == 0) dst[w] = '\n';
+}
+
 // ---------------------------------------------------------------------------
 // The scan kernel.
 // ---------------------------------------------------------------------------
@@ -1818,12 +1845,18 @@ inline unsigned tail_blocks(unsigned long long n_tiles, uint32_t tpb) { return (
 
 // The rows' copy: each block takes its `tiles_per_block` tiles: per-tile prefixes by a
 // block scan, then the block's rows, in order.  Whole lines are copied a row a
-// group of lanes.  Rows of values are short, so they take a thread each, which
+// group of lanes.  Rows of values take a thread each while they are short, which
 // puts its bytes into shared memory; the block then writes the batch's rows,
 // which are contiguous in the output, in whole words.  (768 MB of access-log
 // lines, 6% of them selected: 66 us with a group of lanes a row, 43 so; a warp
-// a row, a tile's rows one after another, took 198.)
+// a row, a tile's rows one after another, took 198.)  Rows of JSON longer than
+// kEmitOwn, and all of a batch that does not fit, are written by groups of lanes
+// too.  (Rows of 100 bytes, 96 MB of them: a thread a row, unstaged, 985 us, so
+// 417; of 1,000 bytes 1,420 and 394.  64 or 256 in kEmitOwn's place measure the
+// same; 16 KB of kEmitStage, with half the blocks in flight, 854 and 404.)
+// A CSV row's cells are a thread's, staged or not: their quoting is a byte's work.
 constexpr uint32_t kEmitStage = 8192;  // bytes of a batch of rows kept in shared memory
+constexpr uint32_t kEmitOwn = 128;     // longest row a thread writes there by itself
 
 template <bool kMixed>
 __global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep, const __grid_constant__ DevPlan plan) {
@@ -1875,8 +1908,9 @@ __global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep, const
       if (kMixed) {
         const DevPlan &P = ep.plans[ep.in_plan[ep.tile_input[t0 + i]]];
         if (P.output_kind != 0 || P.csv_mode) {
+          if (!P.csv_mode) emit_row_group(P, line, (const uint32_t *)(rr + 1), ep.out + at, g);
+          else if (g == 0) emit_row(P, line, h, (const uint32_t *)(rr + 1), ep.out + at);
           if (g == 0) {
-            emit_row(P, line, h, (const uint32_t *)(rr + 1), ep.out + at);
             ep.row_off[row0 + r] = at;
             ep.line_idx[row0 + r] = s_line[i] + h.ordinal;
           }
@@ -1896,7 +1930,7 @@ __global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep, const
 #pragma unroll 1
   for (uint32_t r0 = 0; r0 < rows; r0 += kEmitThreads) {
     const uint32_t r = r0 + threadIdx.x;
-    RowRec h;
+    RowRec h = {};
     const uint32_t *fl = nullptr;
     unsigned long long at = 0;
     if (r < rows) {
@@ -1915,8 +1949,21 @@ __global__ void __launch_bounds__(kEmitThreads) k_rows_emit(EmitParams ep, const
     const unsigned long long b0 = s_span[0], b1 = s_span[1];
     const uint32_t lead = (uint32_t)((uintptr_t)(ep.out + b0) & 3u);
     const bool staged = b1 - b0 + 4 <= kEmitStage;
-    if (r < rows)
-      emit_row(plan, ep.data + h.line_start, h, fl, staged ? s_out + lead + (uint32_t)(at - b0) : ep.out + at);
+    uint8_t *const dst = staged ? s_out + lead + (uint32_t)(at - b0) : ep.out + at;
+    const bool mine = plan.csv_mode || (staged && h.row_len <= kEmitOwn);
+    if (r < rows && mine) emit_row(plan, ep.data + h.line_start, h, fl, dst);
+    if (!plan.csv_mode) {  // the others by groups of lanes, each group its own lanes' rows
+      const uint32_t g = threadIdx.x % kEmitLanes;
+      const unsigned todo = __ballot_sync(0xffffffffu, r < rows && !mine);
+#pragma unroll 1
+      for (uint32_t k = 0; k < kEmitLanes && todo; k++) {
+        const uint32_t from = (threadIdx.x & 31u) - g + k;
+        const unsigned long long line = __shfl_sync(0xffffffffu, h.line_start, from);
+        const uint32_t *const ffl = (const uint32_t *)__shfl_sync(0xffffffffu, (unsigned long long)fl, from);
+        uint8_t *const fdst = (uint8_t *)__shfl_sync(0xffffffffu, (unsigned long long)dst, from);
+        if (todo >> from & 1u) emit_row_group(plan, ep.data + line, ffl, fdst, g);
+      }
+    }
     __syncthreads();
     if (staged) {
       uint8_t *const w0 = ep.out + b0 - lead;  // a word boundary
