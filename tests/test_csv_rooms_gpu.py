@@ -1,0 +1,48 @@
+"""CSV rows where the converter's way of taking them changes: rows around the
+edge of its windows among shorter ones, and rows too long for any window side by
+side."""
+
+import random
+
+import numpy as np
+import pytest
+
+from oracle import csv_map
+
+pytestmark = pytest.mark.gpu
+
+
+def convert(data):
+    import torch
+    import warpjq_b200 as wjq
+    from warpjq_b200.shard import _DeviceBytes
+    dev = torch.from_numpy(np.frombuffer(data, dtype=np.uint8).copy()).cuda()
+    c = wjq.CsvConverter()
+    d, n, used, rows = c.convert(dev.data_ptr(), len(data), stream=torch.cuda.current_stream().cuda_stream)
+    assert used == len(data)
+    out = bytes(torch.as_tensor(_DeviceBytes(d, max(1, n)), device="cuda").cpu().numpy()[:n])
+    c.close()
+    return out
+
+
+def body(rng, n, kind):
+    x = bytes(rng.choices(b"abcdefgh .:;", k=n))
+    if kind == "quoted":
+        x = b'"' + x.replace(b"e", b'""').replace(b".", b",").replace(b":", b"\n") + b'"'
+    elif kind == "control":
+        x = x.replace(b"a", b"\x01").replace(b"b", b"\t")
+    return x
+
+
+@pytest.mark.parametrize("short, long", [(8, [990, 1000, 1005, 1008, 1009, 1010, 1020, 1024, 1100]), (8, [4000, 6000]),
+                                         (100, [3900, 4080, 4096, 4100]), (300, [5090, 5104, 5105, 5119, 5121]),
+                                         (2000, [1200, 1300, 7000]), (9000, [9000, 20]), (6000, [1270, 1275, 1280, 4000])])
+@pytest.mark.parametrize("kind", ["plain", "quoted", "control"])
+def test_rows_among_shorter_ones(short, long, kind):
+    rng = random.Random(short + len(kind))
+    rows = [b"a,b,c"]
+    for i in range(400 if short < 1000 else 130):
+        n = rng.choice(long) + rng.randrange(3) - 8 if rng.randrange(9) == 0 else max(1, short - 4)
+        rows.append(b"%d,%s,%d" % (i, body(rng, n, kind), i % 7))
+    data = b"\n".join(rows) + b"\n"
+    assert convert(data) == csv_map.csv_to_ndjson(data)

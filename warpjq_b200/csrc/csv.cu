@@ -413,11 +413,23 @@ __device__ __forceinline__ uint32_t row_line(const uint8_t *w, const uint32_t *s
   return odd ? 0u : empty ? 1u : len;
 }
 
+// A row by row_json over global memory, out of line: the rows of the windows
+// lose registers to it otherwise (64 MB of rows of 600 bytes: 357 us inline, 333 so).
+template <bool kWrite>
+__device__ __noinline__ u64 row_far(const uint8_t *d, u64 s, u64 e, KeySet ks, uint8_t *to) {
+  WordIn in(d);
+  WordOut wo(to);
+  const u64 len = row_json<kWrite>(in, s, e, ks, wo);
+  if (kWrite) wo.flush();
+  return len;
+}
+
 // Rows [row0, rows) of the chunk: pass 0 writes the NDJSON length of line r -
 // row0 to len_off, pass 1 writes the line at out + len_off[r - row0] (len_off
 // by then an exclusive prefix, *total the end of the last line).  A warp takes
-// as many of its 32 rows at once as fit the staged windows; a row that fits
-// none alone, or has bytes after a closing quote, goes by row_json.
+// as many of its 32 rows at once as fit the staged windows, after those that fit
+// none alone, which go by row_json all at once (one after another, 64 MB of rows
+// of 8,000 bytes took 34.7 ms; 5.2 so).
 template <bool kWrite>
 __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *row_end, u64 row0, u64 rows, KeySet ks,
                                                  u64 *len_off, uint8_t *out, const u64 *total) {
@@ -439,67 +451,63 @@ __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *ro
         o1 = r + 1 < rows ? len_off[r + 1 - row0] : *total;
       }
     }
+    // Rows too long for the windows go by row_json, each lane its own, and with
+    // them those that a window holds few of.
+    bool big = mine && (e - s + 15 >= kCsvWin || (kWrite && o1 - o0 + 15 > kCsvOut));
+    if (__any_sync(0xffffffffu, big)) big = big || (mine && 4 * (e - s) >= kCsvWin);
+    if (big) {
+      const u64 len = row_far<kWrite>(d, s, e, ks, kWrite ? out + o0 : nullptr);
+      if (!kWrite) len_off[r - row0] = len;
+    }
+    const unsigned gone = __ballot_sync(0xffffffffu, big);
     for (uint32_t lo = 0; lo < n_here;) {
+      if (gone >> lo & 1u) {
+        lo++;
+        continue;
+      }
       const u64 s_lo = __shfl_sync(0xffffffffu, s, lo), o_lo = __shfl_sync(0xffffffffu, o0, lo);
       const u64 w0 = (u64)((uintptr_t)(d + s_lo) & 15u);  // the window starts at a block
       const uint32_t lead = (uint32_t)((uintptr_t)(out + o_lo) & 15u);
-      const bool fits = mine && lane >= lo && e - s_lo + w0 < kCsvWin && (!kWrite || o1 - o_lo + lead <= kCsvOut);
+      const bool fits = mine && !big && lane >= lo && e - s_lo + w0 < kCsvWin && (!kWrite || o1 - o_lo + lead <= kCsvOut);
       const unsigned m = __ballot_sync(0xffffffffu, fits) >> lo;
-      const uint32_t take = m == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~m) - 1u;  // rows lo .. lo + take fit
+      const uint32_t take = m == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~m) - 1u;  // rows lo .. lo + take fit, one at least
       const bool on = fits && lane < lo + take;
-      if (take) {
-        const uint32_t hi = lo + take - 1;
-        const uint32_t n_win = (uint32_t)(__shfl_sync(0xffffffffu, e, hi) - s_lo + w0);
-        const uint4 *src = (const uint4 *)((uintptr_t)(d + s_lo) & ~(uintptr_t)15);
-        // whole blocks, each holding a byte of the rows
-        for (uint32_t k = lane; 16 * k < n_win; k += 32) ((uint4 *)win)[k] = __ldg(src + k);
-        __syncwarp();
-        if (lane == 0) win[n_win] = '\n';  // ends the last row
-        __syncwarp();
-        for (uint32_t k = lane; 32 * k <= n_win; k += 32) {
-          const uint4 u = ((const uint4 *)win)[2 * k], v = ((const uint4 *)win)[2 * k + 1];
-          const uint32_t w8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
-          mask[k] = csv_hits(w8);
-        }
-        __syncwarp();
-        const uint32_t ws = on ? (uint32_t)(s - s_lo + w0) : 0u, we = on ? (uint32_t)(e - s_lo + w0) : 0u;
-        const uint32_t at = on ? (uint32_t)(o0 - o_lo) + lead : 0u;
-        LineOut o(obuf, at);
-        uint32_t len = row_line<kWrite>(win, mask, ws, we, on, ks, o);
-        if (on && !len) {  // row_json takes it
-          WordIn in(d);
-          WordOut wo(kWrite ? (uint8_t *)obuf + at : nullptr);
-          len = (uint32_t)row_json<kWrite>(in, s, e, ks, wo);
-          if (kWrite) wo.flush();
-        }
-        __syncwarp();
-        if (!kWrite) {
-          if (on) len_off[r - row0] = len;
-        } else {
-          // whole blocks, and the bytes around them
-          const uint32_t end = (uint32_t)(__shfl_sync(0xffffffffu, o1, hi) - o_lo) + lead;
-          uint8_t *dst = out + o_lo - lead;
-          for (uint32_t k = 16 * lane; k < end; k += 512) {
-            if (k >= lead && k + 16 <= end) {
-              *(uint4 *)(dst + k) = *(const uint4 *)((const uint8_t *)obuf + k);
-            } else {
-              for (uint32_t j = max(k, lead); j < min(k + 16, end); j++) dst[j] = ((const uint8_t *)obuf)[j];
-            }
-          }
-          __syncwarp();
-        }
-        lo += take;
-      } else {  // row lo is too long for the windows
-        if (lane == lo) {
-          WordIn in(d);
-          WordOut wo(kWrite ? out + o0 : nullptr);
-          const u64 len = row_json<kWrite>(in, s, e, ks, wo);
-          if (kWrite) wo.flush();
-          else len_off[r - row0] = len;
-        }
-        __syncwarp();
-        lo++;
+      const uint32_t hi = lo + take - 1;
+      const uint32_t n_win = (uint32_t)(__shfl_sync(0xffffffffu, e, hi) - s_lo + w0);
+      const uint4 *src = (const uint4 *)((uintptr_t)(d + s_lo) & ~(uintptr_t)15);
+      // whole blocks, each holding a byte of the rows
+      for (uint32_t k = lane; 16 * k < n_win; k += 32) ((uint4 *)win)[k] = __ldg(src + k);
+      __syncwarp();
+      if (lane == 0) win[n_win] = '\n';  // ends the last row
+      __syncwarp();
+      for (uint32_t k = lane; 32 * k <= n_win; k += 32) {
+        const uint4 u = ((const uint4 *)win)[2 * k], v = ((const uint4 *)win)[2 * k + 1];
+        const uint32_t w8[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+        mask[k] = csv_hits(w8);
       }
+      __syncwarp();
+      const uint32_t ws = on ? (uint32_t)(s - s_lo + w0) : 0u, we = on ? (uint32_t)(e - s_lo + w0) : 0u;
+      const uint32_t at = on ? (uint32_t)(o0 - o_lo) + lead : 0u;
+      LineOut o(obuf, at);
+      uint32_t len = row_line<kWrite>(win, mask, ws, we, on, ks, o);
+      if (on && !len) len = (uint32_t)row_far<kWrite>(d, s, e, ks, kWrite ? (uint8_t *)obuf + at : nullptr);
+      __syncwarp();
+      if (!kWrite) {
+        if (on) len_off[r - row0] = len;
+      } else {
+        // whole blocks, and the bytes around them
+        const uint32_t end = (uint32_t)(__shfl_sync(0xffffffffu, o1, hi) - o_lo) + lead;
+        uint8_t *dst = out + o_lo - lead;
+        for (uint32_t k = 16 * lane; k < end; k += 512) {
+          if (k >= lead && k + 16 <= end) {
+            *(uint4 *)(dst + k) = *(const uint4 *)((const uint8_t *)obuf + k);
+          } else {
+            for (uint32_t j = max(k, lead); j < min(k + 16, end); j++) dst[j] = ((const uint8_t *)obuf)[j];
+          }
+        }
+        __syncwarp();
+      }
+      lo += take;
     }
   }
 }
