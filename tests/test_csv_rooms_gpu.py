@@ -1,6 +1,6 @@
 """CSV rows where the converter's way of taking them changes: rows around the
 edge of its windows among shorter ones, and rows too long for any window side by
-side."""
+side; bytes after a field's closing quote."""
 
 import random
 
@@ -44,5 +44,19 @@ def test_rows_among_shorter_ones(short, long, kind):
     for i in range(400 if short < 1000 else 130):
         n = rng.choice(long) + rng.randrange(3) - 8 if rng.randrange(9) == 0 else max(1, short - 4)
         rows.append(b"%d,%s,%d" % (i, body(rng, n, kind), i % 7))
+    data = b"\n".join(rows) + b"\n"
+    assert convert(data) == csv_map.csv_to_ndjson(data)
+
+
+@pytest.mark.parametrize("pad", [0, 1, 2, 3, 40, 1500])
+def test_bytes_after_a_closing_quote(pad):
+    x = b"p" * pad
+    tails = [b"z", b'"', b'y"y', b"\\", b"\x02", b"\t\t", b"q" * 50, b' "mid" ', b'""""'[:3], b"a\\b\"c\x01d"]
+    rows = [b"a,b,c"]
+    for t in tails:
+        for inner in (b"", b"in", b'""', b"a,b", b"l\n", b"\\"):
+            if (t.count(b'"') % 2):
+                t = t + b'"'  # quotes stay even within a row
+            rows += [b'%s"%s"%s,2,%s' % (b"", inner + x, t, x), b'1,"%s"%s' % (inner, t), b'"%s"%s,"%s"%s,3' % (inner, t, x, t)]
     data = b"\n".join(rows) + b"\n"
     assert convert(data) == csv_map.csv_to_ndjson(data)

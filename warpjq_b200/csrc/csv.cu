@@ -323,15 +323,14 @@ struct LineOut {
 };
 
 // One row w[s, e) of a window (hits in sm; w[e] is a hit): its NDJSON length,
-// and with kWrite its bytes.  0 for a row with bytes after a field's closing
-// quote, which row_json takes.  The fields' rules are row_json's.
+// and with kWrite its bytes.  The fields' rules are row_json's.
 template <bool kWrite>
 __device__ __forceinline__ uint32_t row_line(const uint8_t *w, const uint32_t *sm, uint32_t s, uint32_t e, bool on,
                                              const KeySet &ks, LineOut &o) {
   if (on && e > s && w[e - 1] == '\r') e--;
   const bool empty = e == s;
   uint32_t len = 3, p = s;  // "{" "}\n"
-  bool more = on && !empty, odd = false;
+  bool more = on && !empty;
   if (kWrite && more) o.put('{', 1);
 #pragma unroll 1
   for (uint32_t k = 0; k < ks.n && __any_sync(0xffffffffu, more); k++) {
@@ -376,32 +375,43 @@ __device__ __forceinline__ uint32_t row_line(const uint8_t *w, const uint32_t *s
     __syncwarp();
     if (more) {
       p = quoted && b < e ? b + 1 : b;  // past the closing quote
-      if (quoted && p < e && w[p] != ',') odd = true;
+      // bytes after it, kept up to the next ',': [p, t)
+      uint32_t t = p;
+      if (quoted)
+#pragma unroll 1
+        while (t < e && w[t] != ',') {
+          const uint32_t h = min(wjq::detail::next_special(sm, t), e);
+          if (h < e && w[h] != ',') extra += esc_len(w[h]) - 1;
+          t = h + (h < e && w[h] != ',');
+        }
       const bool null = !quoted && b == a;
       const bool number = !quoted && !esc && !null && (c == '-' || c - '0' < 10u) && wjq::detail::win_number(w, a, c) == b;
       const bool str = !null && !number;
-      len += null ? 4u : b - a + extra + (str ? 2u : 0u);
+      len += null ? 4u : b - a + (t - p) + extra + (str ? 2u : 0u);
       if (kWrite) {
         if (null) o.put('n' | 'u' << 8 | 'l' << 16 | (uint32_t)'l' << 24, 4);
         if (str) o.put('"', 1);
-        uint32_t q = a;
+        auto escaped = [&](uint32_t q, uint32_t end, bool doubled) {
 #pragma unroll 1
-        while (esc && q < b) {
-          const uint32_t h = min(wjq::detail::next_special(sm, q), b);
-          o.copy(w, q, h);
-          q = h;
-          if (h < b) {
-            const uint32_t x = w[h];
-            if (x == ',') o.put(',', 1);
-            else o.escape(x);
-            q += x == '"' && quoted ? 2 : 1;
+          while (q < end) {
+            const uint32_t h = min(wjq::detail::next_special(sm, q), end);
+            o.copy(w, q, h);
+            q = h;
+            if (h < end) {
+              const uint32_t x = w[h];
+              if (x == ',') o.put(',', 1);
+              else o.escape(x);
+              q += x == '"' && doubled ? 2 : 1;
+            }
           }
-        }
-        if (!esc && !null) o.copy(w, a, b);
+        };
+        if (esc) escaped(a, b, quoted);
+        else if (!null) o.copy(w, a, b);
+        if (t > p) escaped(p, t, false);
         if (str) o.put('"', 1);
       }
-      more = p < e && !odd;  // a ',' follows
-      p++;
+      more = t < e;  // a ',' follows
+      p = t + 1;
     }
     __syncwarp();
   }
@@ -410,7 +420,7 @@ __device__ __forceinline__ uint32_t row_line(const uint8_t *w, const uint32_t *s
     else o.put('}' | '\n' << 8, 2);
     o.flush();
   }
-  return odd ? 0u : empty ? 1u : len;
+  return empty ? 1u : len;
 }
 
 // A row by row_json over global memory, out of line: the rows of the windows
@@ -489,8 +499,7 @@ __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *ro
       const uint32_t ws = on ? (uint32_t)(s - s_lo + w0) : 0u, we = on ? (uint32_t)(e - s_lo + w0) : 0u;
       const uint32_t at = on ? (uint32_t)(o0 - o_lo) + lead : 0u;
       LineOut o(obuf, at);
-      uint32_t len = row_line<kWrite>(win, mask, ws, we, on, ks, o);
-      if (on && !len) len = (uint32_t)row_far<kWrite>(d, s, e, ks, kWrite ? (uint8_t *)obuf + at : nullptr);
+      const uint32_t len = row_line<kWrite>(win, mask, ws, we, on, ks, o);
       __syncwarp();
       if (!kWrite) {
         if (on) len_off[r - row0] = len;
