@@ -1,6 +1,6 @@
-"""CSV rows where the converter's way of taking them changes: rows around the
-edge of its windows among shorter ones, and rows too long for any window side by
-side; bytes after a field's closing quote."""
+"""CSV rows where the converter's way of taking them changes: windows sized for
+short rows with rows around their edge among them, rows too long for any window
+side by side; bytes after a field's closing quote."""
 
 import random
 
@@ -34,6 +34,7 @@ def body(rng, n, kind):
     return x
 
 
+# the smallest window is 1,024 bytes, the largest 5,120 (8,192 for the lines)
 @pytest.mark.parametrize("short, long", [(8, [990, 1000, 1005, 1008, 1009, 1010, 1020, 1024, 1100]), (8, [4000, 6000]),
                                          (100, [3900, 4080, 4096, 4100]), (300, [5090, 5104, 5105, 5119, 5121]),
                                          (2000, [1200, 1300, 7000]), (9000, [9000, 20]), (6000, [1270, 1275, 1280, 4000])])

@@ -240,12 +240,21 @@ __global__ void k_csv_close(u64 *row_end, u64 n, int final_, u64 *info) {
 // of windows leave 15 warps an SM, and the lanes' escapes fall on different
 // bytes.  (Copying short pieces byte by byte took 857, byte by byte through
 // the fields with escapes 938.)
-constexpr uint32_t kCsvWin = 5120;   // staged input bytes
-constexpr uint32_t kCsvOut = 8192;   // staged output bytes
-constexpr uint32_t kCsvMask = kCsvWin / 32 + 2;
-constexpr uint32_t kCsvOff = kCsvWin + 64 + (kCsvMask * 4 + 15) / 16 * 16;  // where the output starts
+constexpr uint32_t kCsvWin = 5120;   // staged input bytes, at most
+constexpr uint32_t kCsvOut = 8192;   // staged output bytes, at most
 
-__host__ __device__ constexpr uint32_t csv_smem(bool write) { return kCsvOff + (write ? kCsvOut + 16 : 0u); }
+// The windows of one launch: room for 32 rows of the average length and a
+// quarter, so that short rows leave shared memory for more warps (64 MB of rows
+// of 30 bytes: 562 us with the largest windows, 434 so).
+struct CsvWin {
+  uint32_t in, out;  // bytes; out 0: no output is staged
+  __host__ __device__ uint32_t mask_words() const { return (in / 32 + 2 + 3) & ~3u; }
+  __host__ __device__ uint32_t out_at() const { return in + 64 + mask_words() * 4; }
+  __host__ __device__ uint32_t smem() const { return out_at() + (out ? out + 16 : 0u); }
+};
+uint32_t csv_room(u64 bytes, u64 rows, uint32_t most) {
+  return (uint32_t)std::min<u64>(most, std::max<u64>(1024, (40 * bytes / rows + 127) & ~(u64)31));
+}
 
 // The hits of eight words: ',' '"' '\\' and bytes below 0x20 (devutil.cuh
 // flags_special, with ',').
@@ -442,11 +451,11 @@ __device__ __noinline__ u64 row_far(const uint8_t *d, u64 s, u64 e, KeySet ks, u
 // of 8,000 bytes took 34.7 ms; 5.2 so).
 template <bool kWrite>
 __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *row_end, u64 row0, u64 rows, KeySet ks,
-                                                 u64 *len_off, uint8_t *out, const u64 *total) {
+                                                 u64 *len_off, uint8_t *out, const u64 *total, CsvWin room) {
   extern __shared__ __align__(16) uint8_t csv_sm[];
   uint8_t *win = csv_sm;
-  uint32_t *mask = (uint32_t *)(csv_sm + kCsvWin + 64);
-  uint32_t *obuf = (uint32_t *)(csv_sm + kCsvOff);
+  uint32_t *mask = (uint32_t *)(csv_sm + room.in + 64);
+  uint32_t *obuf = (uint32_t *)(csv_sm + room.out_at());
   const uint32_t lane = threadIdx.x;
   for (u64 base = row0 + blockIdx.x * 32ull; base < rows; base += gridDim.x * 32ull) {
     const u64 r = base + lane;
@@ -463,8 +472,8 @@ __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *ro
     }
     // Rows too long for the windows go by row_json, each lane its own, and with
     // them those that a window holds few of.
-    bool big = mine && (e - s + 15 >= kCsvWin || (kWrite && o1 - o0 + 15 > kCsvOut));
-    if (__any_sync(0xffffffffu, big)) big = big || (mine && 4 * (e - s) >= kCsvWin);
+    bool big = mine && (e - s + 15 >= room.in || (kWrite && o1 - o0 + 15 > room.out));
+    if (__any_sync(0xffffffffu, big)) big = big || (mine && 4 * (e - s) >= room.in);
     if (big) {
       const u64 len = row_far<kWrite>(d, s, e, ks, kWrite ? out + o0 : nullptr);
       if (!kWrite) len_off[r - row0] = len;
@@ -478,7 +487,7 @@ __global__ void __launch_bounds__(32) k_csv_json(const uint8_t *d, const u64 *ro
       const u64 s_lo = __shfl_sync(0xffffffffu, s, lo), o_lo = __shfl_sync(0xffffffffu, o0, lo);
       const u64 w0 = (u64)((uintptr_t)(d + s_lo) & 15u);  // the window starts at a block
       const uint32_t lead = (uint32_t)((uintptr_t)(out + o_lo) & 15u);
-      const bool fits = mine && !big && lane >= lo && e - s_lo + w0 < kCsvWin && (!kWrite || o1 - o_lo + lead <= kCsvOut);
+      const bool fits = mine && !big && lane >= lo && e - s_lo + w0 < room.in && (!kWrite || o1 - o_lo + lead <= room.out);
       const unsigned m = __ballot_sync(0xffffffffu, fits) >> lo;
       const uint32_t take = m == 0xFFFFFFFFu ? 32u : (uint32_t)__ffs(~m) - 1u;  // rows lo .. lo + take fit, one at least
       const bool on = fits && lane < lo + take;
@@ -729,7 +738,8 @@ warpjq_status warpjq_csv_convert(warpjq_csv *c, const uint8_t *src, uint64_t n, 
   KeySet ks{c->keys.p, c->key_off.p, (uint32_t)(c->key_meta.size() / 2)};
   CSV_CK(c->lens.ensure(m + 1), "device memory for CSV lines");
   const unsigned grid = (unsigned)std::min<u64>((m + 31) / 32, 148ull * 256);
-  k_csv_json<false><<<grid, 32, csv_smem(false), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, nullptr, nullptr);
+  CsvWin room{csv_room(n, rows, kCsvWin), 0};
+  k_csv_json<false><<<grid, 32, room.smem(), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, nullptr, nullptr, room);
   const u64 nb = (m + kScanBlock - 1) / kScanBlock;
   CSV_CK(c->bt.ensure(nb), "device memory for CSV lines");
   k_sum_blocks<<<(unsigned)nb, 256, 0, st>>>(c->lens.p, m, c->bt.p);
@@ -740,8 +750,9 @@ warpjq_status warpjq_csv_convert(warpjq_csv *c, const uint8_t *src, uint64_t n, 
   CSV_CK(cudaMemcpyAsync(&total, c->info.p + 3, 8, cudaMemcpyDeviceToHost, st), "CSV line lengths");
   CSV_CK(cudaStreamSynchronize(st), "CSV line lengths");
   CSV_CK(c->out.ensure(total + 16), "device memory for the NDJSON");
-  k_csv_json<true><<<grid, 32, csv_smem(true), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, c->out.p,
-                                                     c->info.p + 3);
+  room.out = csv_room(total, m, kCsvOut);
+  k_csv_json<true><<<grid, 32, room.smem(), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, c->out.p,
+                                                  c->info.p + 3, room);
   CSV_CK(cudaGetLastError(), "CSV to NDJSON");
   *d_ndjson = c->out.p;
   *ndjson_len = total;
