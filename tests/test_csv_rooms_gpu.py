@@ -1,6 +1,7 @@
 """CSV rows where the converter's way of taking them changes: windows sized for
 short rows with rows around their edge among them, rows too long for any window
-side by side; bytes after a field's closing quote."""
+side by side, lines of many columns (written a lane a row), and bytes after a
+field's closing quote."""
 
 import random
 
@@ -47,6 +48,21 @@ def test_rows_among_shorter_ones(short, long, kind):
         rows.append(b"%d,%s,%d" % (i, body(rng, n, kind), i % 7))
     data = b"\n".join(rows) + b"\n"
     assert convert(data) == csv_map.csv_to_ndjson(data)
+
+
+@pytest.mark.parametrize("columns", [8, 9, 20, 60])
+@pytest.mark.parametrize("width", [0, 1, 4, 7, 30, 90])
+def test_many_columns(columns, width):
+    rng = random.Random(columns * 100 + width)
+    rows = [b",".join(b"name_%d" % k for k in range(columns))]
+    for i in range(150):
+        n = rng.randrange(columns + 2) if i % 5 == 0 else columns
+        cell = lambda: rng.choice([b"%d" % rng.randrange(10**max(1, min(width, 9))), bytes(rng.choices(b"xy z", k=width)),
+                                   b"", b'"' + b"q" * width + b'"', b'"a""b"' if width > 3 else b"7"])
+        rows.append(b",".join(cell() for _ in range(n)))
+    for end in (b"\n", b"\r\n"):
+        data = end.join(rows)
+        assert convert(data) == csv_map.csv_to_ndjson(data)
 
 
 @pytest.mark.parametrize("pad", [0, 1, 2, 3, 40, 1500])

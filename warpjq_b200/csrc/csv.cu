@@ -245,7 +245,8 @@ constexpr uint32_t kCsvOut = 8192;   // staged output bytes, at most
 
 // The windows of one launch: room for 32 rows of the average length and a
 // quarter, so that short rows leave shared memory for more warps (64 MB of rows
-// of 30 bytes: 562 us with the largest windows, 434 so).
+// of 30 bytes: 562 us with the largest windows, 434 so).  Both 0: every row goes
+// by row_json.
 struct CsvWin {
   uint32_t in, out;  // bytes; out 0: no output is staged
   __host__ __device__ uint32_t mask_words() const { return (in / 32 + 2 + 3) & ~3u; }
@@ -254,6 +255,17 @@ struct CsvWin {
 };
 uint32_t csv_room(u64 bytes, u64 rows, uint32_t most) {
   return (uint32_t)std::min<u64>(most, std::max<u64>(1024, (40 * bytes / rows + 127) & ~(u64)31));
+}
+
+// Whether lines are better written by row_json, a lane a row over global memory.
+// With fewer rows in a window than lanes, what the windows save at each field's
+// bytes is lost on the lanes that wait through its steps.  Measured on 64 MB,
+// the windows against row_json, us: 50 columns of 7 bytes, lines of 950 bytes
+// 1,373 and 897; 30 of 25 bytes, lines of 1,000, 855 and 551; 40 of 3 bytes,
+// lines of 430, 957 and 689; 10 of 3 bytes, lines of 110, 533 and 673; 4 of 75
+// bytes 308 and 486, of 250 bytes 359 and 743.
+bool csv_direct(u64 in, u64 out, u64 rows, u64 columns) {
+  return columns > 8 && out > rows * (in < 6 * columns * rows ? 320u : 560u);
 }
 
 // The hits of eight words: ',' '"' '\\' and bytes below 0x20 (devutil.cuh
@@ -751,6 +763,7 @@ warpjq_status warpjq_csv_convert(warpjq_csv *c, const uint8_t *src, uint64_t n, 
   CSV_CK(cudaStreamSynchronize(st), "CSV line lengths");
   CSV_CK(c->out.ensure(total + 16), "device memory for the NDJSON");
   room.out = csv_room(total, m, kCsvOut);
+  if (csv_direct(n, total, m, ks.n)) room.in = room.out = 0;
   k_csv_json<true><<<grid, 32, room.smem(), st>>>(d, c->row_end.p, row0, rows, ks, c->lens.p, c->out.p,
                                                   c->info.p + 3, room);
   CSV_CK(cudaGetLastError(), "CSV to NDJSON");
