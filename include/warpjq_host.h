@@ -69,7 +69,8 @@ int warpjq_run_bytes(const char *query, const uint8_t *data, size_t len, uint32_
                      char **out, size_t *out_len, uint64_t *stats, char *err, size_t err_len);
 
 /* Formats a device-resident aggregate result; `data` is a host copy of the
- * input (group keys are rendered from it). */
+ * input (group keys are rendered from it).  Nonzero, with *out null, when
+ * memory runs out. */
 int warpjq_query_render_device(warpjq_query *q, const warpjq_device_result *r,
                                const uint8_t *data, char **out, size_t *out_len);
 

@@ -495,8 +495,10 @@ class Query:
             addr = ctypes.cast(keep, ctypes.c_void_p)
         else:
             addr = ctypes.c_void_p(host_data.ctypes.data)
-        self._h.warpjq_query_render_device(self._q, ctypes.byref(r), addr, ctypes.byref(out),
-                                           ctypes.byref(n))
+        rc = self._h.warpjq_query_render_device(self._q, ctypes.byref(r), addr, ctypes.byref(out),
+                                                ctypes.byref(n))
+        if rc:
+            raise MemoryError("rendering the result")
         return _take(out, n)
 
 

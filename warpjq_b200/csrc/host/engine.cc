@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <atomic>
 #include <condition_variable>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <cerrno>
@@ -359,7 +360,9 @@ struct Writer {
   void device_groups(const std::string &name, uint32_t kind, const uint8_t *data, const warpjq_group_ext *gs,
                      uint32_t n);
   // Hands the output to the caller as one malloc'd, NUL-terminated buffer.
+  // Null when memory ran out for it, or for any part before.
   char *finish(size_t &len) {
+    if (oom) return nullptr;
     if (fmt == WARPJQ_FMT_COUNT) buf = std::to_string(rows) + "\n";
     if (bulk_rows.p) {
       if (!buf.empty()) oom |= !bulk_rows.append(buf.data(), buf.size());
@@ -393,19 +396,32 @@ struct GroupRow {
   }
 };
 
-// f(0) .. f(n - 1), each on a thread of its own (the last on this one).
+// f(0) .. f(n - 1), each on a thread of its own (the last on this one).  An
+// exception out of one of them is thrown here, once all have returned.
 template <class F>
 void on_threads(unsigned n, F &&f) {
+  std::exception_ptr thrown;
+  std::mutex mu;
+  auto guarded = [&](unsigned t) {
+    try {
+      f(t);
+    } catch (...) {
+      std::lock_guard<std::mutex> lk(mu);
+      if (!thrown) thrown = std::current_exception();
+    }
+  };
   std::vector<std::thread> ws;
+  ws.reserve(n);
   for (unsigned t = 0; t + 1 < n; t++) {
     try {
-      ws.emplace_back(f, t);
-    } catch (const std::system_error &) {  // no thread to be had
-      f(t);
+      ws.emplace_back(std::ref(guarded), t);
+    } catch (const std::exception &) {  // no thread to be had, or no memory for one
+      guarded(t);
     }
   }
-  f(n - 1);
+  guarded(n - 1);
   for (auto &w : ws) w.join();
+  if (thrown) std::rethrow_exception(thrown);
 }
 
 // The groups of a device-resident result in output order.  From 16,384 groups
@@ -1288,15 +1304,21 @@ static void render_head(const warpjq_query *q, Writer &w, uint64_t count, uint64
 // render group keys.
 int warpjq_query_render_device(warpjq_query *q, const warpjq_device_result *r, const uint8_t *data,
                                char **out, size_t *out_len) {
-  Writer w;
-  render_head(q, w, r->count, r->numeric, r->sum, r->min, r->max, r->groups, r->n_groups, r->n_selected,
-              data);
-  size_t res_len = 0;
-  char *res = w.finish(res_len);
-  if (!res) return 1;
-  *out = res;
-  if (out_len) *out_len = res_len;
-  return 0;
+  *out = nullptr;
+  if (out_len) *out_len = 0;
+  try {
+    Writer w;
+    render_head(q, w, r->count, r->numeric, r->sum, r->min, r->max, r->groups, r->n_groups, r->n_selected,
+                data);
+    size_t res_len = 0;
+    char *res = w.finish(res_len);
+    if (!res) return 1;
+    *out = res;
+    if (out_len) *out_len = res_len;
+    return 0;
+  } catch (const std::exception &) {  // out of memory
+    return 1;
+  }
 }
 
 // Every input's output of a collected batch (warpjq_batch_collect), back to
@@ -1309,30 +1331,34 @@ int warpjq_query_render_batch(warpjq_query *q, const warpjq_batch_item *items, u
                               const uint64_t *row_off, char **out, size_t *out_len, uint64_t *offsets) {
   *out = nullptr;
   if (out_len) *out_len = 0;
-  std::string all;
   offsets[0] = 0;
-  for (uint32_t i = 0; i < n; i++) {
-    const warpjq_batch_item &it = items[i];
-    Writer w;
-    render_head(q, w, it.count, it.numeric, it.sum, it.min, it.max, groups ? groups + it.group_begin : nullptr,
-                it.n_groups, it.n_selected, key_data);
-    size_t hl = 0;
-    char *h = w.finish(hl);
-    if (!h) return 1;
-    all.append(h, hl);
-    free(h);
-    if (it.n_selected && rows && row_off) {
-      const uint64_t a = row_off[it.row_begin], b = row_off[it.row_begin + it.n_selected];
-      all.append((const char *)rows + a, b - a);
+  try {
+    std::string all;
+    for (uint32_t i = 0; i < n; i++) {
+      const warpjq_batch_item &it = items[i];
+      Writer w;
+      render_head(q, w, it.count, it.numeric, it.sum, it.min, it.max, groups ? groups + it.group_begin : nullptr,
+                  it.n_groups, it.n_selected, key_data);
+      size_t hl = 0;
+      char *h = w.finish(hl);
+      if (!h) return 1;
+      std::unique_ptr<char, decltype(&free)> held(h, &free);
+      all.append(h, hl);
+      if (it.n_selected && rows && row_off) {
+        const uint64_t a = row_off[it.row_begin], b = row_off[it.row_begin + it.n_selected];
+        all.append((const char *)rows + a, b - a);
+      }
+      offsets[i + 1] = all.size();
     }
-    offsets[i + 1] = all.size();
+    char *res = (char *)malloc(all.size() + 1);
+    if (!res) return 1;
+    memcpy(res, all.data(), all.size());
+    *out = res;
+    if (out_len) *out_len = all.size();
+    return 0;
+  } catch (const std::exception &) {  // out of memory
+    return 1;
   }
-  char *res = (char *)malloc(all.size() + 1);
-  if (!res) return 1;
-  memcpy(res, all.data(), all.size());
-  *out = res;
-  if (out_len) *out_len = all.size();
-  return 0;
 }
 
 }  // extern "C"
