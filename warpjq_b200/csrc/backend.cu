@@ -155,6 +155,17 @@ __global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, Temp
 // Context.
 // ---------------------------------------------------------------------------
 
+constexpr size_t kFirstGroups = 64;         // group results that come along with the counters
+constexpr size_t kHostGroups = 8192;        // first page-locked room for more (0.7 MB)
+constexpr size_t kPinnedGroups = 1u << 20;  // which grows up to this (92 MB)
+
+// What a run always hands the host, in one page-locked piece.
+struct HostHead {
+  RunCounters ctr;  // mirror of the last run's counters
+  warpjq_group_ext ext[kFirstGroups];
+  uint32_t in[kFirstGroups];
+};
+
 struct Slot {
   cudaStream_t stream = nullptr;
   cudaEvent_t done = nullptr;
@@ -162,8 +173,8 @@ struct Slot {
   uint8_t *d_chunk = nullptr;
   unsigned long long n_bytes = 0;
   RunBufs rb;
-  RunCounters *h_ctr = nullptr;  // pinned mirror of the last run's counters
-  bool mirrored = false;         // the last run's kernels write it
+  HostHead *h_head = nullptr;
+  bool mirrored = false;  // the last run's kernels write h_head->ctr
   // pinned result mirrors
   std::vector<uint8_t> dummy;
   uint8_t *h_out = nullptr;
@@ -174,10 +185,12 @@ struct Slot {
   size_t h_rows_cap = 0;
   warpjq_group *h_groups = nullptr;
   size_t h_groups_cap = 0;
-  // group results copied from the device: page-locked up to kPinnedGroups
+  // more than kFirstGroups group results copied from the device: page-locked
+  // from the second such result on, up to kPinnedGroups
   warpjq_group_ext *h_ext = nullptr;
   uint32_t *h_in = nullptr;
   size_t h_ext_cap = 0;
+  bool many_groups = false;
   std::vector<warpjq_group_ext> v_ext;
   std::vector<uint32_t> v_in;
   bool launched = false;
@@ -531,7 +544,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     tp.row_tiles = rows ? rb.row_tiles.p : nullptr;
     tp.bsum = rb.row_bsum.p;
     tp.ctr = rb.ctr.p;
-    tp.mirror = s.h_ctr;
+    tp.mirror = &s.h_head->ctr;
     tp.row_off = rb.row_off.p;
     tp.rows_cap = rb.rows_cap;
     tp.out_cap = rb.out_cap;
@@ -626,10 +639,6 @@ bool grow_after_overflow(warpjq_ctx *c, Slot &s, const RunCounters &h, unsigned 
   return again;
 }
 
-constexpr size_t kFirstGroups = 64;          // copied with the counters
-constexpr size_t kHostGroups = 8192;         // first page-locked room (0.7 MB), taken with a grouped context
-constexpr size_t kPinnedGroups = 1u << 20;  // page-locked room for results grows up to this (92 MB)
-
 warpjq_status ensure_host_groups(Slot &s, size_t n, char *err, size_t err_len) {
   if (n <= s.h_ext_cap) return WARPJQ_OK;
   if (s.h_ext) cudaFreeHost(s.h_ext);
@@ -637,8 +646,8 @@ warpjq_status ensure_host_groups(Slot &s, size_t n, char *err, size_t err_len) {
   s.h_ext = nullptr;
   s.h_in = nullptr;
   s.h_ext_cap = 0;
-  // Page-locking and releasing memory stalls the whole device, so a slot does
-  // it seldom: from kHostGroups on, at least doubling.
+  // Page-locking and releasing memory takes long and stalls the whole device,
+  // so a slot does it seldom: from kHostGroups on, at least doubling.
   const size_t cap = std::max(n, std::min(std::max(2 * n, kHostGroups), kPinnedGroups));
   CK(cudaHostAlloc((void **)&s.h_ext, cap * sizeof(warpjq_group_ext), cudaHostAllocDefault), "pinned groups");
   CK(cudaHostAlloc((void **)&s.h_in, cap * sizeof(uint32_t), cudaHostAllocDefault), "pinned groups");
@@ -657,16 +666,14 @@ warpjq_status run_to_completion(warpjq_ctx *c, Slot &s, const uint8_t *d_data,
       if (rc != WARPJQ_OK) return rc;
     }
     if (!s.mirrored)
-      CK(cudaMemcpyAsync(s.h_ctr, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st), "D2H counters");
+      CK(cudaMemcpyAsync(&s.h_head->ctr, s.rb.ctr.p, sizeof(RunCounters), cudaMemcpyDeviceToHost, st),
+         "D2H counters");
     if (run_grouped(c, b)) {  // few groups come along, without a second wait
-      warpjq_status rc = ensure_host_groups(s, kFirstGroups, err, err_len);
-      if (rc != WARPJQ_OK) return rc;
-      CK(cudaMemcpyAsync(s.h_ext, s.rb.g_ext.p, kFirstGroups * sizeof(warpjq_group_ext), cudaMemcpyDeviceToHost, st),
-         "D2H groups");
-      if (b) CK(cudaMemcpyAsync(s.h_in, s.rb.g_in.p, kFirstGroups * 4, cudaMemcpyDeviceToHost, st), "D2H groups");
+      CK(cudaMemcpyAsync(s.h_head->ext, s.rb.g_ext.p, sizeof(s.h_head->ext), cudaMemcpyDeviceToHost, st), "D2H groups");
+      if (b) CK(cudaMemcpyAsync(s.h_head->in, s.rb.g_in.p, sizeof(s.h_head->in), cudaMemcpyDeviceToHost, st), "D2H groups");
     }
     CK(cudaStreamSynchronize(st), "stream sync");
-    h = *s.h_ctr;
+    h = s.h_head->ctr;
     if (h.error) {
       set_err(err, err_len, "the scan kernel raised its error flag");
       return WARPJQ_ERR_CUDA;
@@ -794,7 +801,7 @@ warpjq_status warpjq_ctx_create(const warpjq_program *prog, uint64_t max_chunk_b
     CK(cudaHostAlloc((void **)&s.h_chunk, std::max<uint64_t>(max_chunk_bytes, 16), cudaHostAllocDefault),
        "pinned chunk");
     CK(cudaMalloc((void **)&s.d_chunk, max_chunk_bytes + 16), "device chunk");
-    CK(cudaHostAlloc((void **)&s.h_ctr, sizeof(RunCounters), cudaHostAllocDefault), "pinned ctr");
+    CK(cudaHostAlloc((void **)&s.h_head, sizeof(HostHead), cudaHostAllocDefault), "pinned counters");
     if (max_chunk_bytes) {
       rc = ensure_bufs(c.get(), s, max_chunk_bytes, (max_chunk_bytes + c->tile_bytes - 1) / c->tile_bytes,
                        s.stream, false, err, err_len, run_grouped(c.get(), nullptr), run_rows(c.get(), nullptr),
@@ -803,11 +810,7 @@ warpjq_status warpjq_ctx_create(const warpjq_program *prog, uint64_t max_chunk_b
       CK(cudaStreamSynchronize(s.stream), "stream sync");
     }
   }
-  CK(cudaHostAlloc((void **)&c->dev.h_ctr, sizeof(RunCounters), cudaHostAllocDefault), "pinned ctr");
-  if (run_grouped(c.get(), nullptr)) {
-    rc = ensure_host_groups(c->dev, kHostGroups, err, err_len);
-    if (rc != WARPJQ_OK) return rc;
-  }
+  CK(cudaHostAlloc((void **)&c->dev.h_head, sizeof(HostHead), cudaHostAllocDefault), "pinned counters");
   *out = c.release();
   return WARPJQ_OK;
 }
@@ -818,7 +821,7 @@ static void free_slot(Slot &s) {
   if (s.done) cudaEventDestroy(s.done);
   if (s.h_chunk) cudaFreeHost(s.h_chunk);
   if (s.d_chunk) cudaFree(s.d_chunk);
-  if (s.h_ctr) cudaFreeHost(s.h_ctr);
+  if (s.h_head) cudaFreeHost(s.h_head);
   if (s.h_out) cudaFreeHost(s.h_out);
   if (s.h_row_off) cudaFreeHost(s.h_row_off);
   if (s.h_line64) cudaFreeHost(s.h_line64);
@@ -944,10 +947,12 @@ static warpjq_status fetch_groups(Slot &s, const RunCounters &h, cudaStream_t st
                                   const warpjq_group_ext *&gs, const uint32_t *&gin, size_t &n, char *err,
                                   size_t err_len) {
   n = h.n_groups;
-  warpjq_group_ext *ext = s.h_ext;
-  uint32_t *in = s.h_in;
+  warpjq_group_ext *ext = s.h_head->ext;
+  uint32_t *in = s.h_head->in;
   if (n > kFirstGroups) {
-    if (n > kPinnedGroups) {
+    // A first result through pageable memory costs less than locking room for
+    // it, which a query that runs once would not use again.
+    if (n > kPinnedGroups || !s.many_groups) {
       s.v_ext.resize(n);
       s.v_in.resize(inputs ? n : 0);
       ext = s.v_ext.data();
@@ -955,9 +960,12 @@ static warpjq_status fetch_groups(Slot &s, const RunCounters &h, cudaStream_t st
     } else {
       warpjq_status rc = ensure_host_groups(s, n, err, err_len);
       if (rc != WARPJQ_OK) return rc;
+      std::vector<warpjq_group_ext>().swap(s.v_ext);
+      std::vector<uint32_t>().swap(s.v_in);
       ext = s.h_ext;
       in = s.h_in;
     }
+    s.many_groups = true;
     CK(cudaMemcpyAsync(ext, s.rb.g_ext.p, n * sizeof(warpjq_group_ext), cudaMemcpyDeviceToHost, st), "D2H groups");
     if (inputs) CK(cudaMemcpyAsync(in, s.rb.g_in.p, n * 4, cudaMemcpyDeviceToHost, st), "D2H groups");
     CK(cudaStreamSynchronize(st), "stream sync");
