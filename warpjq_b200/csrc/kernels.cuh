@@ -1007,6 +1007,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
     if (lane == 0 && win_reaches_end) win[wlen] = '\n';  // ends the last line for the walker
     if (tstate < kTmplReady) {
       tstate = __shfl_sync(0xffffffffu, tsee, 0);
+      __syncwarp();  // the other lanes' reads come after lane 0's acquire (a tile under 16 bytes has no copy to wait for)
       if (tstate == kTmplReady)
 #pragma unroll 1
         for (uint32_t k = lane; k < sizeof(Template) / 4; k += 32)
@@ -1203,7 +1204,7 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
               if (lane == __ffs(ok) - 1 && atomicCAS(&sp.tmpl->state, kTmplNone, kTmplBuilding) == kTmplNone) {
                 uint32_t next = kTmplReady;
                 if (!build_template(P, win, smask, s, e, tmpl))
-                  next = ++sp.tmpl->tries < kTmplTries ? kTmplNone : kTmplOff;
+                  next = atomicAdd(&sp.tmpl->tries, 1u) + 1u < kTmplTries ? kTmplNone : kTmplOff;  // CTAs take turns at it
                 else
                   sp.tmpl->t = *tmpl;
                 __threadfence();
