@@ -424,16 +424,19 @@ void on_threads(unsigned n, F &&f) {
   if (thrown) std::rethrow_exception(thrown);
 }
 
-// The groups of a device-resident result in output order.  From 16,384 groups
+// The groups of a device-resident result in output order.  From 4,096 groups
 // on the work is split over up to 16 threads (reading the keys, all over the
 // input; splitting them into ranges of the output order by a sample; sorting
 // and printing each range): 150,000 groups took 54 ms as one sort of
-// key strings, 3 ms so; below, threads cost more than they save.
+// key strings, 3 ms so.  Starting threads for the four rounds takes some 0.9 ms
+// of 16 cores; one thread against 16: 2,048 groups 0.66 and 1.01 ms, 4,096 1.43
+// and 1.16, 8,192 3.14 and 1.44, 16,384 6.73 and 2.01 (8 slower cores: 2,048
+// 1.76 and 1.08).
 void Writer::device_groups(const std::string &name, uint32_t kind, const uint8_t *data, const warpjq_group_ext *gs,
                            uint32_t n) {
   rows += n;
   if (fmt == WARPJQ_FMT_COUNT || !n) return;
-  const unsigned T = n < 16384 ? 1u : std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
+  const unsigned T = n < 4096 ? 1u : std::min(16u, std::max(1u, std::thread::hardware_concurrency()));
   auto part = [&](unsigned t) { return (uint32_t)((uint64_t)n * t / T); };
   std::vector<GroupRow> in(n), out(T > 1 ? n : 0);
   std::vector<std::vector<std::unique_ptr<std::string>>> decoded(T);  // keys with escapes
