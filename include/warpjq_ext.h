@@ -166,7 +166,7 @@ warpjq_status warpjq_batch_launch(warpjq_ctx *ctx, const uint8_t *d_data, const 
  * input_ctx[i], so inputs with different queries share one launch sequence:
  * one launch of the persistent scan per distinct query, each over the tiles
  * of that query's inputs with its plan as a kernel parameter, then one set
- * of row, reduce and finalize passes.  Aggregate and row queries alike; each
+ * of tail, row and finalize passes.  Aggregate and row queries alike; each
  * input's rows are a contiguous range of the batch's output, in input
  * order.  `ctx` supplies the buffers, tiling and stream order, and is
  * collected with warpjq_batch_collect; each item is then rendered by its own

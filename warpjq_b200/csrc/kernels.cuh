@@ -101,7 +101,7 @@ __host__ __device__ inline size_t scan_smem_base(uint32_t T, uint32_t H) {
   return (s + 15) & ~(size_t)15;
 }
 
-// Record of one selected row, staged per CTA until the look-back resolves.
+// Record of one selected row, appended to the CTA's record arena for k_rows_emit.
 struct RowRec {
   unsigned long long line_start;  // absolute offset of the line
   uint32_t line_len;              // without '\n' and without a trailing '\r'
@@ -180,7 +180,7 @@ static_assert(sizeof(GroupKeyDesc) == 24, "group key descriptor");
 constexpr uint32_t kKeyCache = 32;       // one lane clears one
 constexpr uint32_t kKeyCacheBytes = 24;  // longest key kept
 constexpr uint32_t kKeyAccBytes = 2048;
-constexpr uint32_t kFoldLines = 32768;   // 65,535 of them could overflow lo
+constexpr uint32_t kFoldLines = 32768;   // lo, 65,535 a line at most, holds 65,537
 struct KeyCache {
   uint32_t hash[kKeyCache];  // 0: free
   uint32_t meta[kKeyCache];  // length | kind << 24

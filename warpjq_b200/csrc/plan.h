@@ -132,10 +132,11 @@ struct RunCounters {
   // counts units of 2^(32 k - 128); values of magnitude >= 2^128 go to fbig
   long long fix[8];
   double fbig;
-  double fsum_total;         // written by the finalize kernel: the rounded fix sum + fbig
-  double sum_total;          // written by the finalize kernel: integer + fix sums rounded once, + fbig
-  unsigned long long first_invalid;     // written by the finalize kernel
-  unsigned long long first_type_error;  // written by the finalize kernel
+  // written by k_tail, and for a batch's inputs by k_batch_finalize
+  double fsum_total;         // the rounded fix sum + fbig
+  double sum_total;          // integer + fix sums rounded once, + fbig
+  unsigned long long first_invalid;
+  unsigned long long first_type_error;
 };
 
 }  // namespace wjq
