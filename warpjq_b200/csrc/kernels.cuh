@@ -43,8 +43,9 @@ constexpr int kThreads = 32;                 // one warp per CTA; each warp owns
 constexpr uint32_t kMaxLinesPerPass = 128;   // line-start list capacity per pass
 // Register budgets of k_scan (CTAs of one warp per SM), measured per variant
 // on 1 GB of the nginx workload: the ungrouped aggregate at 20 (96 registers,
-// 8 bytes of spills: 685 us; at 24, with 144 bytes, 713; at 16, 775), the row
-// variant at 20 and the group-by variant at 16 (128).  What the warps have in
+// then 8 bytes of spills: 685 us; at 24, with 144 bytes, 713; at 16, 775; since
+// wide tiles note their lines too, 52 bytes and 702 us), the row variant at 20
+// and the group-by variant at 16 (128).  What the warps have in
 // common is the instruction cache: the body's loops are kept rolled and the
 // rare walks out of line, which took the same scan from 840 us to 685 with the
 // same work (misses had kept the next cache level 56% busy; 34% then).
