@@ -56,3 +56,20 @@ def test_more_than_page_locked_room():
         want = b"".join(b'{"k":%d,"sum":%d}\n' % (i, 2 * i + n) for i in range(n))
         assert q.render_device(r, data) == want
     q.close()
+
+
+def test_collected_again():
+    """A run's groups stay where they were handed out until the next launch."""
+    import ctypes
+    import torch
+    import warpjq_b200 as wjq
+    data = lines(3000)
+    dev = torch.from_numpy(np.frombuffer(data + b"\0" * 16, dtype=np.uint8).copy()).cuda()
+    q = wjq.Query("group_by(.k) | sum(.v)", chunk_bytes=1 << 20)
+    for _ in range(3):
+        q.launch_device(dev.data_ptr(), len(data), torch.cuda.current_stream().cuda_stream)
+        a, b = q.collect_device(), q.collect_device()
+        at = [ctypes.cast(r.groups, ctypes.c_void_p).value for r in (a, b)]
+        assert at[0] == at[1] and a.n_groups == b.n_groups == 3000
+        assert q.render_device(a, data) == orc.run("group_by(.k) | sum(.v)", data).out
+    q.close()

@@ -190,7 +190,8 @@ struct Slot {
   warpjq_group_ext *h_ext = nullptr;
   uint32_t *h_in = nullptr;
   size_t h_ext_cap = 0;
-  bool many_groups = false;
+  bool many_groups = false;  // a run before this one had more
+  bool more_groups = false;  // a collected run had more
   std::vector<warpjq_group_ext> v_ext;
   std::vector<uint32_t> v_in;
   bool launched = false;
@@ -437,6 +438,7 @@ warpjq_status enqueue_run(warpjq_ctx *c, Slot &s, const uint8_t *d_data, unsigne
     CK(cudaEventRecord(s.btab_done, st), "event record");
   }
   s.kernels = 0;
+  s.many_groups = s.more_groups;
   s.mirrored = n > 0 && n_tiles > 0;
   if (b && n_inputs) {
     k_batch_reset<<<(n_inputs + 255) / 256, 256, 0, st>>>(rb.b_in_ctr.p, n_inputs);
@@ -951,7 +953,8 @@ static warpjq_status fetch_groups(Slot &s, const RunCounters &h, cudaStream_t st
   uint32_t *in = s.h_head->in;
   if (n > kFirstGroups) {
     // A first result through pageable memory costs less than locking room for
-    // it, which a query that runs once would not use again.
+    // it, which a query that runs once would not use again.  (A run collected
+    // again goes the same way: what it handed out stays.)
     if (n > kPinnedGroups || !s.many_groups) {
       s.v_ext.resize(n);
       s.v_in.resize(inputs ? n : 0);
@@ -965,7 +968,7 @@ static warpjq_status fetch_groups(Slot &s, const RunCounters &h, cudaStream_t st
       ext = s.h_ext;
       in = s.h_in;
     }
-    s.many_groups = true;
+    s.more_groups = true;
     CK(cudaMemcpyAsync(ext, s.rb.g_ext.p, n * sizeof(warpjq_group_ext), cudaMemcpyDeviceToHost, st), "D2H groups");
     if (inputs) CK(cudaMemcpyAsync(in, s.rb.g_in.p, n * 4, cudaMemcpyDeviceToHost, st), "D2H groups");
     CK(cudaStreamSynchronize(st), "stream sync");
@@ -1531,6 +1534,7 @@ warpjq_status warpjq_batch_graph_launch(warpjq_batch_graph *g, void *stream, cha
     c->batch.active = true;
     c->batch.stream = st;
     c->dev.launched = true;
+    c->dev.many_groups = c->dev.more_groups;
     c->dev.mirrored = g->mirrored[i];
     c->dev.timed = false;
     c->dev.kernels = g->kernels[i];
