@@ -143,7 +143,7 @@ __global__ void k_reset_run(RunCounters *ctr, GroupTable g, uint32_t g_cap, Temp
     z.first_invalid = ~0ull;
     *ctr = z;
   }
-  for (unsigned long long i = tid; i < n_tmpl; i += stride) tmpl[i].state = tmpl[i].tries = 0;
+  for (unsigned long long i = tid; i < n_tmpl; i += stride) tmpl[i].state = tmpl[i].tries = tmpl[i].misses = 0;
   if (g.slots) {
     for (unsigned long long i = tid; i < g_cap; i += stride) g.slots[i] = 0;
   }

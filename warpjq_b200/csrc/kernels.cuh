@@ -222,11 +222,20 @@ struct RowTile {
 struct TemplateBuf {
   uint32_t state;  // kTmpl*, set to kTmplNone before the run
   uint32_t tries;  // lines that had no template
+  uint32_t misses;  // rounds that missed a line by it
   Template t;
 };
 constexpr uint32_t kTmplNone = 0, kTmplBuilding = 1, kTmplReady = 2, kTmplOff = 3;
 constexpr uint32_t kTmplTries = 4;   // lines tried before the run goes on without one
 constexpr uint32_t kTmplMisses = 3;  // rounds that missed a line, past every second one, before a CTA stops using it
+// The run gives the template up when more than kTmplDrop tenths of its rounds
+// miss a line: such a round walks the template and the line, with the other
+// lanes waiting.  k_scan, us, of 600 MB of access-log lines with an optional
+// member in some: never given up 0.5% of the lines (15% of the rounds) 518, 1%
+// (28%) 562, 2% (48%) 629, 5% (81%) 723; no template 570 to 580.  (Each CTA by
+// itself needed some ten rounds to see it: 648 at 2%, 642 at 5%; so 588 and 589.)
+constexpr uint32_t kTmplDrop = 3;
+constexpr uint32_t kTmplFirst = 64;  // rounds that may miss before that
 
 struct ScanParams {
   const uint8_t *data;
@@ -896,6 +905,18 @@ __device__ __noinline__ unsigned long long far_newline(const uint8_t *d, unsigne
   return q;
 }
 
+// One more round missed a line by the template, in a tile of n_lines lines:
+// whether the run is better off without it.  `next` is the CTA's next ticket.
+__device__ __noinline__ bool template_missed(TemplateBuf *t, unsigned long long next, uint32_t n_lines) {
+  const unsigned long long m = atomicAdd(&t->misses, 1u) + 1ull;
+  if (*(volatile uint32_t *)&t->state == kTmplOff) return true;
+  // tiles walked by it: all that are taken, but every CTA's first and next
+  const unsigned long long taken = 2ull * gridDim.x, tiles = next > taken ? next - taken : 0ull;
+  if (10 * m <= 10 * kTmplFirst + kTmplDrop * tiles * ((n_lines + 31u) >> 5)) return false;
+  atomicExch(&t->state, kTmplOff);
+  return true;
+}
+
 // The plan is a kernel parameter (constant bank): fields at fixed offsets
 // are instruction operands, and no plan read goes through global memory.
 // kGroups: the group-by path is compiled in (grouped aggregates); without
@@ -1195,8 +1216,11 @@ __global__ void __launch_bounds__(kThreads, kGroups ? kScanBlocksPerSMGrouped : 
           __syncwarp();
           const unsigned ok = __ballot_sync(0xffffffffu, walk && status == LS_OK);
           if (tstate == kTmplReady) {
-            // a template that most rounds miss a line of costs more than it saves
-            if (ok && (tmisses += 2) > 2 * kTmplMisses) tstate = kTmplOff;
+            // a template that many rounds miss a line of costs more than it saves
+            if (ok) {
+              const bool off = lane == 0 && template_missed(sp.tmpl, next_ticket, n_lines_tile);
+              if (__any_sync(0xffffffffu, off) || (tmisses += 2) > 2 * kTmplMisses) tstate = kTmplOff;
+            }
           } else if (tstate == kTmplNone) {
             // one line is enough, and only a CTA with another tile to walk tries
             const bool more = __shfl_sync(0xffffffffu, next_ticket < n_work ? 1u : 0u, 0);
